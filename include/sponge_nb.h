@@ -442,12 +442,8 @@ int snb_engine_profile_steps(snb_engine* e, float* crd, float* vel,
  * shape, times `steps` replays of the captured step graph (stream-launched
  * steps for the pair search's shape, or where the stream is the legacy
  * default one), each from the given coordinates, and keeps the fastest:
- * the pair kernel's candidates per lane per scan round (2, 4, 8) and
- * persistent blocks per SM (occupancy maximum, 2, 3), its rows in flight
- * per block (4, 8, 16 warps for one box, 8 or 16 for a batch; plain LJ),
- * whether its hit list keeps each hit's displacement, charge and LJ pair
- * index in shared memory (so that the pair terms gather nothing; plain
- * single box, at most 4 candidates per lane), the pair search's
+ * the pair kernel's persistent blocks per SM (occupancy maximum, 2, 3, in
+ * blocks of 512 threads), the pair search's
  * blocks per SM (4, 8, 16), the PME gather's threads per block (128, 256,
  * 512), the PME spread's shape (tiles of edge 8 with 1, 2, 4 warps per
  * tile, or edge 0: int64 global atomics, no tiles; single box; edge 16 with
@@ -463,7 +459,9 @@ int snb_engine_profile_steps(snb_engine* e, float* crd, float* vel,
  * recaptures the step graph.  h_choice[0..8] receives {unroll, blocks per
  * SM (0 = occupancy maximum), search blocks per SM, gather threads, pair
  * warps per block, spread tile edge, spread warps per tile, hit stash (0 /
- * 1), own FFT (0 / 1)}.  Allocates scratch. */
+ * 1), own FFT (0 / 1)}; unroll, pair warps and the hit stash belong to
+ * earlier pair kernels: they are kept as set and change nothing.  Allocates
+ * scratch. */
 int snb_engine_autotune(snb_engine* e, float* crd, float* vel,
                         const float* inverse_mass, float dt, int steps,
                         int* h_choice, void* stream);
@@ -488,15 +486,14 @@ int snb_engine_stats(snb_engine* e, long long* rebuilds, long long* pairs,
  * with the atomics no tile is taken again and the count stays 0. */
 int snb_engine_spread_wide_tiles(snb_engine* e, int* count, void* stream);
 /* The engine's neighbor list holds the pair set of NEIGHBOR_LIST::Update
- * (neighbor_list.cpp:974-1025) in one of two forms.  Rows (the default):
- * one row of partners per atom, as snb_nl keeps them.  Clusters (on request,
- * for one rectangular box of at least five cells per axis, not with the
- * soft-core kernel): runs of up to four atoms of a cell, and per cluster
- * the clusters with a pair within cutoff + skin, each with its 4x4 pair
- * mask; the pair kernel loads a neighbour cluster once for four atoms.
- * Both hold the same pairs.  clusters = 0 / 1 picks the form (1 is refused
- * where the box or the soft-core kernel does not allow it); the next step
- * rebuilds the list. */
+ * (neighbor_list.cpp:974-1025) as grouped rows: runs of up to eight atoms of
+ * a cell, and per group the atoms with a pair within cutoff + skin, which the
+ * pair kernel loads once for the whole group.  clusters = 0 / 1 chose between
+ * two earlier forms of the list; both values now give the grouped rows.  The
+ * value is kept for snb_engine_list_form, 1 is refused where that form was
+ * (a batch, a box below five cells per axis, the soft-core kernel), and the
+ * next step rebuilds the list.  (Float accumulation, and boxes of 2^24 atoms
+ * or more, keep a row of partners per atom, as snb_nl does.) */
 int snb_engine_set_list_form(snb_engine* e, int clusters);
 /* Virtual atoms in the engine (NULL to remove): every force evaluation moves
  * the sites' forces onto their atoms before the forces are returned or the
@@ -504,21 +501,21 @@ int snb_engine_set_list_form(snb_engine* e, int clusters);
  * (and before the first step).  The sites' inverse masses must be 0. */
 int snb_engine_set_virtual_atoms(snb_engine* e, snb_vatom* vatom);
 int snb_engine_list_form(snb_engine* e, int* clusters);
-/* No counterpart in the reference.  Pruned rows for the plain LJ rows of a
- * single box: a prune pass of the pair kernel scans the full rows (the
- * entries within cutoff + skin) and keeps those within cutoff + margin; the
- * steps after it scan only the kept entries, until an atom has moved more
- * than half the margin since the pass or the list is rebuilt.  A pair
- * outside cutoff + margin at the pass stays outside the cutoff until then,
- * so every step sees the same pairs within the cutoff as without pruning
- * and the forces are the same bit for bit.  snb_engine_create (for boxes of
- * at least 20,000 atoms) and snb_batch_create set a margin of 0.8 A;
- * margin 0 turns it off.  Force
- * calls outside the MD steps always scan the full rows.  Not used with the
- * cluster form. */
+/* No counterpart in the reference.  Pruned rows: a prune pass of the pair
+ * kernel takes the full rows and notes, for every 32 entries of a row, which
+ * of the group's atoms have a partner among them within cutoff + margin; the
+ * steps after it take only those, until an atom has moved more than half the
+ * margin since the pass or the list is rebuilt.  A pair outside cutoff +
+ * margin at the pass stays outside the cutoff until then, so every step sees
+ * the same pairs within the cutoff as without pruning and the forces are the
+ * same bit for bit.  snb_engine_create (for boxes of at least 20,000 atoms)
+ * and snb_batch_create set a margin of 0.8 A; margin 0 turns it off.  Force
+ * calls outside the MD steps always take the full rows.  No effect with float
+ * accumulation. */
 int snb_engine_set_prune_margin(snb_engine* e, float margin);
-/* Prune passes run so far, and (kept_entries may be null) the entries the
- * last pass kept in all rows (host sync; 0 while pruning was never on). */
+/* Prune passes run so far, and (kept_entries may be null) the entries of all
+ * rows that lie in the 32s the last pass kept (host sync; 0 while pruning was
+ * never on). */
 int snb_engine_prune_passes(snb_engine* e, int* passes, long long* kept_entries,
                             void* stream);
 /* The engine's current pair set in global ids, lo < hi, in no particular

@@ -156,13 +156,22 @@ struct snb_engine {
   snb_vatom* vatom = nullptr;    // massless sites: forces moved, positions refreshed
   long long* d_nb14_sums = nullptr;  // [2]
   double* d_kin = nullptr;           // [6] scratch of the pressure call
-  // launch shapes picked by snb_engine_autotune
+  // grouped-row pair kernel (fixed point): the {A', B'} tables and the packed
+  // types (caller frame) of the plain LJ and of the soft-core module in use
+  float2* d_lj_tab = nullptr;
+  int* d_gtype = nullptr;
+  float2* d_soft_a = nullptr;
+  float2* d_soft_b = nullptr;
+  int* d_soft_type = nullptr;
+  bool cluster_form = false;    // what snb_engine_list_form reports
+  // launch shapes: blocks per SM is tuned; the others are settings of pair
+  // kernels that are gone, kept for callers that set and read them back
   int pair_unroll = 4;
   int pair_blocks_per_sm = 0;
-  int pair_warps = 16;  // measured on the 100k box: 4 candidates x 16 rows is the fastest
+  int pair_warps = 16;
   bool pair_stash = false;
-  // pruned rows (single box, plain LJ rows): between prune passes the pair
-  // kernel scans only the entries within cutoff + prune_margin (0: off).
+  // pruned rows: between prune passes the pair kernel takes only the parts
+  // of the rows within cutoff + prune_margin (0: off).
   // d_prune = {pass this step, an atom moved more than half the margin since
   // the last pass, list generation at the last pass, passes so far}
   float prune_margin = 0.f;
@@ -207,7 +216,7 @@ constexpr float kDefaultPruneMargin = 0.8f;  // A
 constexpr int kPruneMinAtoms = 20000;        // single boxes below: full rows
 
 static bool engine_prunes(const snb_engine* e) {
-  return e->prune_margin > 0.f && e->d_prune && !(e->nl.clusters && !e->soft);
+  return e->prune_margin > 0.f && e->d_prune && e->nl.groups;
 }
 
 // The check that follows an update: displacements above half the margin
@@ -982,11 +991,96 @@ extern "C" int snb_pme_destroy(snb_pme* h) {
 // ============================================================= engine
 // Everything of engine creation after the neighbor list and PME: LJ tables,
 // charges, exclusions, accumulators and the step scratch.
+// {A', B'} per pair of types as the grouped pair kernel reads them, the full
+// square (a byte offset within it fits 31 bits).
+constexpr int kMaxTypes = 16384;
+static int upload_pair_table(int T, const float* A, const float* B, float2** d) {
+  if (T > kMaxTypes) return fail(kNotSupported, "engine: too many LJ types");
+  std::vector<float2> t((size_t)T * T);
+  for (int a = 0; a < T; ++a)
+    for (int b = 0; b < T; ++b)
+      t[(size_t)a * T + b] = make_float2(A[lj_pair_index(a, b)], B[lj_pair_index(a, b)]);
+  cudaFree(*d);
+  *d = nullptr;
+  SNB_CUDA_TRY(cudaMalloc(d, sizeof(float2) * t.size()));
+  SNB_CUDA_TRY(cudaMemcpy(*d, t.data(), sizeof(float2) * t.size(), cudaMemcpyHostToDevice));
+  return kOk;
+}
+
+// Types whose A' and B' are zero with every type (water H).
+static std::vector<char> types_without_lj(int T, const float* A, const float* B) {
+  std::vector<char> none(T, 1);
+  for (int a = 0; a < T; ++a)
+    for (int b = 0; b <= a; ++b) {
+      const int p = lj_pair_index(a, b);
+      if (A[p] != 0.f || B[p] != 0.f) none[a] = none[b] = 0;
+    }
+  return none;
+}
+
+// The soft-core module's tables and packed types for the grouped pair kernel.
+// An atom is marked (sign bit) unless every pair of unmarked atoms has equal
+// end states, so that a pair of two unmarked atoms takes the plain terms: its
+// (A type, B type) joins the unmarked ones, in order of how many atoms carry
+// it, when its pairs with all of them (and itself) are equal in both states.
+static int engine_soft_tables(snb_engine* e, const snb_lj_soft* h) {
+  const int nA = h->nA, nB = h->nB, n = e->n;
+  const size_t smem = sizeof(float) * ((size_t)nA * (nA + 1) + (size_t)nB * (nB + 1));
+  if (smem > 48 * 1024) return kOk;  // refused when a step runs
+  const int pA = nA * (nA + 1) / 2, pB = nB * (nB + 1) / 2;
+  std::vector<float> AA(pA), AB(pA), BA(pB), BB(pB);
+  std::vector<int2> par(n);
+  SNB_CUDA_TRY(cudaMemcpy(AA.data(), h->d_AA, sizeof(float) * pA, cudaMemcpyDeviceToHost));
+  SNB_CUDA_TRY(cudaMemcpy(AB.data(), h->d_AB, sizeof(float) * pA, cudaMemcpyDeviceToHost));
+  SNB_CUDA_TRY(cudaMemcpy(BA.data(), h->d_BA, sizeof(float) * pB, cudaMemcpyDeviceToHost));
+  SNB_CUDA_TRY(cudaMemcpy(BB.data(), h->d_BB, sizeof(float) * pB, cudaMemcpyDeviceToHost));
+  SNB_CUDA_TRY(cudaMemcpy(par.data(), h->d_par_local, sizeof(int2) * n,
+                          cudaMemcpyDeviceToHost));
+  const std::vector<char> noneA = types_without_lj(nA, AA.data(), AB.data());
+  const std::vector<char> noneB = types_without_lj(nB, BA.data(), BB.data());
+  std::vector<int> count((size_t)nA * nB, 0);
+  for (int i = 0; i < n; ++i) ++count[(par[i].x & 0xffff) * nB + (par[i].x >> 16)];
+  std::vector<int> kinds;
+  for (size_t k = 0; k < count.size(); ++k)
+    if (count[k]) kinds.push_back((int)k);
+  std::stable_sort(kinds.begin(), kinds.end(),
+                   [&](int x, int y) { return count[x] > count[y]; });
+  std::vector<char> marked(count.size(), 1);
+  std::vector<int> plain;
+  for (int k : kinds) {
+    plain.push_back(k);
+    bool equal = true;
+    for (int q : plain) {
+      const int a = lj_pair_index(k / nB, q / nB), b = lj_pair_index(k % nB, q % nB);
+      equal = equal && AA[a] == BA[b] && AB[a] == BB[b];
+    }
+    if (equal)
+      marked[k] = 0;
+    else
+      plain.pop_back();
+  }
+  std::vector<int> packed(n);
+  for (int i = 0; i < n; ++i) {
+    const int tA = par[i].x & 0xffff, tB = par[i].x >> 16;
+    unsigned v = (unsigned)tA | ((unsigned)tB << 15);
+    if (noneA[tA] && noneB[tB]) v |= (unsigned)kTypeNoLJ;
+    if (marked[tA * nB + tB]) v |= 0x80000000u;
+    packed[i] = (int)v;
+  }
+  int rc = upload_pair_table(nA, AA.data(), AB.data(), &e->d_soft_a);
+  if (!rc) rc = upload_pair_table(nB, BA.data(), BB.data(), &e->d_soft_b);
+  if (rc) return rc;
+  if (!e->d_soft_type) SNB_CUDA_TRY(cudaMalloc(&e->d_soft_type, sizeof(int) * n));
+  SNB_CUDA_TRY(cudaMemcpy(e->d_soft_type, packed.data(), sizeof(int) * n,
+                          cudaMemcpyHostToDevice));
+  return kOk;
+}
+
 static int engine_finish_create(snb_engine* e, int n, int n_types, const int* h_type,
                                 const float* h_A, const float* h_B, const float* h_charge,
                                 const int* h_es, const int* h_en, const int* h_el,
                                 int n_excl) {
-  int rc = acc_init(e->acc, n);
+  int rc = acc_init(e->acc, n, e->nl.groups);
   if (rc) return rc;
   LJParams& p = e->lj;
   p.n_types = n_types;
@@ -1021,6 +1115,16 @@ static int engine_finish_create(snb_engine* e, int n, int n_types, const int* h_
   SNB_CUDA_TRY(cudaMemcpy(p.d_B, h_B, sizeof(float) * p.n_pairs, cudaMemcpyHostToDevice));
   SNB_CUDA_TRY(cudaMalloc(&p.d_type, sizeof(int) * n));
   SNB_CUDA_TRY(cudaMemcpy(p.d_type, h_type, sizeof(int) * n, cudaMemcpyHostToDevice));
+  if (e->nl.groups) {
+    const std::vector<char> none = types_without_lj(n_types, h_A, h_B);
+    std::vector<int> packed(n);
+    for (int i = 0; i < n; ++i) packed[i] = h_type[i] | (none[h_type[i]] ? kTypeNoLJ : 0);
+    rc = upload_pair_table(n_types, h_A, h_B, &e->d_lj_tab);
+    if (rc) return rc;
+    SNB_CUDA_TRY(cudaMalloc(&e->d_gtype, sizeof(int) * n));
+    SNB_CUDA_TRY(cudaMemcpy(e->d_gtype, packed.data(), sizeof(int) * n,
+                            cudaMemcpyHostToDevice));
+  }
   SNB_CUDA_TRY(cudaMalloc(&e->d_charge, sizeof(float) * n));
   SNB_CUDA_TRY(cudaMemcpy(e->d_charge, h_charge, sizeof(float) * n, cudaMemcpyHostToDevice));
   SNB_CUDA_TRY(cudaMalloc(&e->d_pos, sizeof(float4) * n));
@@ -1100,7 +1204,7 @@ extern "C" int snb_engine_create(const snb_options* opt, int n, snb_boundary bou
   e->rcell = rcell_of(boundary);
   int rc = nl_init(e->nl, n, e->opt.cutoff, e->opt.skin, boundary.cell,
                    e->opt.nl_refresh_interval, e->opt.nl_skin_permit,
-                   e->opt.nl_max_neighbor_numbers, 0);
+                   e->opt.nl_max_neighbor_numbers, 0, e->accum == kAccumFixed);
   float box[3] = {boundary.cell[0], boundary.cell[2], boundary.cell[5]};
   if (!rc)
     rc = pme_init(e->pme, n, boundary.cell, box, e->opt.cutoff, e->opt.pm_direct_tolerance,
@@ -1116,11 +1220,9 @@ extern "C" int snb_engine_create(const snb_options* opt, int n, snb_boundary bou
     rc = engine_finish_create(e, n, n_types, h_type, h_A, h_B, h_charge, h_es, h_en, h_el,
                               n_excl);
   // pruned rows at 0.8 A: on the 100k box (cutoff 10 A, skin 2 A) a prune
-  // pass every 7-8 steps and the MD step 4 % shorter than with full rows
-  // (0.3 A: 269-275 us, 0.5: 271-272, 0.8: 268-271, 1.2: 273-275; off:
-  // 276-285).  On the 9,000-atom box the extra launch and the passes cost
-  // more than they save (631 against 680 ns/day), so small boxes keep the
-  // full rows.
+  // pass every 7-8 steps, the pair kernel 14 us shorter than with full rows.
+  // On the 9,000-atom box the extra launch and the passes cost what they
+  // save, so small boxes keep the full rows.
   if (!rc && n >= kPruneMinAtoms) rc = snb_engine_set_prune_margin(e, kDefaultPruneMargin);
   if (rc) {
     snb_engine_destroy(e);
@@ -1184,7 +1286,7 @@ extern "C" int snb_batch_create(const snb_options* opt, int n_systems,
   e->rcell = e->h_sys[0].rcell;
   int rc = nl_init_batch(e->nl, n, e->opt.cutoff, e->opt.skin, e->h_sys,
                          e->opt.nl_refresh_interval, e->opt.nl_skin_permit,
-                         e->opt.nl_max_neighbor_numbers);
+                         e->opt.nl_max_neighbor_numbers, true);
   if (!rc)
     rc = pme_init_batch(e->pme, n, e->h_sys, e->opt.cutoff, e->opt.pm_direct_tolerance,
                         e->opt.pm_grid_spacing, e->opt.pme_calculate_reciprocal_part != 0,
@@ -1319,19 +1421,17 @@ static int engine_forces(snb_engine* e, const float* crd, int step, bool energy,
   if (rc) return rc;
   prof_mark(e, 1, st);
   const bool do_pme = e->pme.reciprocal && step % e->pme.update_interval == 0;
-  // cluster form: the pair frame holds each atom in its cell's image
-  const bool clus = e->nl.clusters && !e->soft;
-  const float3* img = clus ? e->nl.d_img_off : nullptr;
+  const bool groups = e->nl.groups;
+  const int* types = !groups ? e->lj.d_type : (e->soft ? e->d_soft_type : e->d_gtype);
+  if (e->soft && (!groups || !types))
+    return fail(kNotSupported, "soft-core rows: type tables too large");
   if (do_pme)
-    rc = pme_pack_bin(e->pme, e->n, reinterpret_cast<const float3*>(crd), e->d_charge,
-                      e->lj.d_type, e->nl.d_perm, e->d_pos, e->d_type_sorted, st, img);
+    rc = pme_pack_bin(e->pme, e->n, reinterpret_cast<const float3*>(crd), e->d_charge, types,
+                      e->nl.d_perm, e->d_pos, e->d_type_sorted, st);
   else
-    rc = launch_pack(e->n, reinterpret_cast<const float3*>(crd), e->d_charge,
-                     e->lj.d_type, e->nl.d_perm, e->d_pos, e->d_type_sorted, st, img);
+    rc = launch_pack(e->n, reinterpret_cast<const float3*>(crd), e->d_charge, types,
+                     e->nl.d_perm, e->d_pos, e->d_type_sorted, st);
   if (rc) return rc;
-  if (e->soft)
-    k_pack_soft<<<ceil_div(e->n, 256), 256, 0, st>>>(e->n, e->nl.d_perm, e->soft->d_par_local,
-                                                    nullptr, e->soft->d_par_sorted, nullptr);
   prof_mark(e, 2, st);
   const bool fork = !e->prof_on;
   cudaStream_t sb = fork ? e->branch : st;
@@ -1359,93 +1459,69 @@ static int engine_forces(snb_engine* e, const float* crd, int step, bool energy,
       return rc;
     SNB_CUDA_TRY(cudaEventRecord(e->ev_join, sb));
   }
-  PairArgs a;
-  a.n = e->n;
-  a.pos = e->d_pos;
-  a.type = e->d_type_sorted;
-  a.global = e->nl.d_global;
-  a.row_start = e->nl.d_row_start;
-  a.row_count = e->nl.d_row_count;
-  a.cols = e->nl.d_cols;
-  a.nl_flags = e->nl.d_flags;
-  a.A = e->lj.d_A;
-  a.B = e->lj.d_B;
-  a.n_types = e->lj.n_types;
-  a.cell = e->cell;
-  a.rcell = e->rcell;
-  a.cutoff2 = e->opt.cutoff * e->opt.cutoff;
-  a.beta = e->pme.beta;
-  a.bv = e->bv;
-  a.unroll = e->pair_unroll;
-  a.blocks_per_sm = e->pair_blocks_per_sm;
-  a.warps = e->pair_warps;
-  a.stash = e->pair_stash;
-  if (engine_prunes(e)) {
-    if (!in_graph) {  // (in the graph the rebuild condition's kernel decides)
-      k_prune_decide<<<1, 1, 0, st>>>(e->d_prune, e->nl.d_flags);
-      SNB_CUDA_TRY(cudaGetLastError());
+  if (groups) {
+    GroupArgs a;
+    a.n = e->n;
+    a.ngroups = e->nl.max_groups;
+    a.group = e->nl.d_group;
+    a.row_count = e->nl.d_grow_count;
+    a.entry = e->nl.d_gentry;
+    a.cap = e->nl.gcap;
+    a.pos = e->d_pos;
+    a.type = e->d_type_sorted;
+    a.nl_flags = e->nl.d_flags;
+    a.lj = e->d_lj_tab;
+    a.n_types = e->lj.n_types;
+    a.cell = e->cell;
+    a.rcell = e->rcell;
+    a.cutoff = e->opt.cutoff;
+    a.cutoff2 = e->opt.cutoff * e->opt.cutoff;
+    a.beta = e->pme.beta;
+    a.bv = e->bv;
+    a.blocks_per_sm = e->pair_blocks_per_sm;
+    if (e->soft) {
+      a.lj = e->d_soft_a;
+      a.n_types = e->soft->nA;
+      a.lj_b = e->d_soft_b;
+      a.n_types_b = e->soft->nB;
+      a.lambda = e->soft->lambda;
+      a.alp_A = e->soft->alpha * powf(e->soft->lambda, e->soft->p);
+      a.alp_B = e->soft->alpha * powf(1.0f - e->soft->lambda, e->soft->p);
+      a.sigma6 = e->soft->sigma6;
+      a.sigma6_min = e->soft->sigma6_min;
     }
-    const float rp = e->opt.cutoff + e->prune_margin;
-    a.prune = e->d_prune;
-    a.cols_in = e->nl.d_cols_in;
-    a.row_in_count = e->nl.d_row_in_count;
-    a.prune_ref = e->nl.d_prune_ref;
-    a.prune2 = rp * rp;
-  } else if ((rc = engine_prune_invalidate(e, st))) {
-    return rc;
-  }
-  if (e->soft) {
-    SoftArgs sa;
-    sa.n = e->n;
-    sa.pos = e->d_pos;
-    sa.par = e->soft->d_par_sorted;
-    sa.dq = nullptr;
-    sa.global = e->nl.d_global;
-    sa.row_start = e->nl.d_row_start;
-    sa.row_count = e->nl.d_row_count;
-    sa.cols = e->nl.d_cols;
-    sa.nl_flags = e->nl.d_flags;
-    sa.AA = e->soft->d_AA;
-    sa.AB = e->soft->d_AB;
-    sa.BA = e->soft->d_BA;
-    sa.BB = e->soft->d_BB;
-    sa.n_types_A = e->soft->nA;
-    sa.n_types_B = e->soft->nB;
-    sa.cell = e->cell;
-    sa.rcell = e->rcell;
-    sa.cutoff2 = a.cutoff2;
-    sa.beta = a.beta;
-    sa.lambda = e->soft->lambda;
-    sa.alpha = e->soft->alpha;
-    sa.p = e->soft->p;
-    sa.sigma6 = e->soft->sigma6;
-    sa.sigma6_min = e->soft->sigma6_min;
-    sa.prune = a.prune;
-    sa.cols_in = a.cols_in;
-    sa.row_in_count = a.row_in_count;
-    sa.prune_ref = a.prune_ref;
-    sa.prune2 = a.prune2;
-    rc = launch_soft_rows(sa, e->acc, energy, virial, st);
-  } else if (clus) {
-    ClusterPairArgs ca;
-    ca.clus = e->nl.d_clus;
-    ca.nclus = e->nl.d_nclus;
-    ca.crow_count = e->nl.d_crow_count;
-    ca.centry = e->nl.d_centry;
-    ca.ccap = e->nl.ccap;
-    ca.pos = e->d_pos;
-    ca.type = e->d_type_sorted;
-    ca.global = e->nl.d_global;
-    ca.nl_flags = e->nl.d_flags;
-    ca.A = e->lj.d_A;
-    ca.B = e->lj.d_B;
-    ca.n_types = e->lj.n_types;
-    ca.box = make_float3(e->cell.a11, e->cell.a22, e->cell.a33);
-    ca.cutoff2 = a.cutoff2;
-    ca.beta = a.beta;
-    ca.blocks_per_sm = e->pair_blocks_per_sm;
-    rc = launch_pair_clusters(ca, e->acc, e->accum, energy, virial, st);
+    if (engine_prunes(e)) {
+      if (!in_graph) {  // (in the graph the rebuild condition's kernel decides)
+        k_prune_decide<<<1, 1, 0, st>>>(e->d_prune, e->nl.d_flags);
+        SNB_CUDA_TRY(cudaGetLastError());
+      }
+      a.prune = e->d_prune;
+      a.mask = e->nl.d_gmask;
+      a.prune_ref = e->nl.d_prune_ref;
+      a.prune_r = e->opt.cutoff + e->prune_margin;
+      a.prune2 = a.prune_r * a.prune_r;
+    } else if ((rc = engine_prune_invalidate(e, st))) {
+      return rc;
+    }
+    rc = launch_pair_groups(a, e->acc, energy, virial, st);
   } else {
+    PairArgs a;
+    a.n = e->n;
+    a.pos = e->d_pos;
+    a.type = e->d_type_sorted;
+    a.global = e->nl.d_global;
+    a.row_start = e->nl.d_row_start;
+    a.row_count = e->nl.d_row_count;
+    a.cols = e->nl.d_cols;
+    a.nl_flags = e->nl.d_flags;
+    a.A = e->lj.d_A;
+    a.B = e->lj.d_B;
+    a.n_types = e->lj.n_types;
+    a.cell = e->cell;
+    a.rcell = e->rcell;
+    a.cutoff2 = e->opt.cutoff * e->opt.cutoff;
+    a.beta = e->pme.beta;
+    a.bv = e->bv;
     rc = launch_pair(a, e->acc, e->accum, energy, virial, true, st);
   }
   if (rc) return rc;
@@ -1714,6 +1790,7 @@ extern "C" int snb_engine_update_box(snb_engine* e, snb_boundary boundary) {
     return fail(kBadInput, "engine_update_box: box lengths must be > 0");
   int rc = nl_regrid(e->nl, c6);
   if (rc) return rc;
+  if (!e->nl.trim) e->cluster_form = false;
   if ((rc = pme_update_box(e->pme, c6))) return rc;
   e->cell = make_cell(c6);
   Cell r{};
@@ -1769,11 +1846,11 @@ extern "C" int snb_engine_set_soft_core(snb_engine* e, snb_lj_soft* soft) {
     if (soft->n != e->n) return fail(kBadInput, "engine_set_soft_core: atom count differs");
   }
   e->soft = soft;
-  // the soft-core pair kernel reads the rows
-  if (soft && e->nl.clusters) {
-    int rc = nl_set_clusters(e->nl, false);
+  if (soft) {
+    e->cluster_form = false;
+    SNB_CUDA_TRY(cudaDeviceSynchronize());  // steps queued with the previous tables
+    const int rc = engine_soft_tables(e, soft);
     if (rc) return rc;
-    e->steps_done = 0;  // the next step rebuilds the list in its new form
   }
   if (soft) {
     const double vol = (double)e->cell.a11 * e->cell.a22 * e->cell.a33;
@@ -2088,8 +2165,8 @@ extern "C" int snb_engine_profile_steps(snb_engine* e, float* crd, float* vel,
 }
 
 // Times `steps` stream-launched steps from the same starting coordinates for
-// each candidate launch shape and keeps the fastest: the pair kernel's scan
-// unroll (2, 4, 8) and blocks per SM (occupancy maximum, 2, 3) by the whole
+// each candidate launch shape and keeps the fastest: the pair kernel's
+// persistent blocks per SM (occupancy maximum, 2, 3) by the whole
 // step (the PME branch shares the SMs with it), the pair
 // search's blocks per SM (4, 8, 16; a rebuild is forced every step), and the
 // gather's threads per block (128, 256, 512).  crd / vel are restored.
@@ -2183,32 +2260,9 @@ extern "C" int snb_engine_autotune(snb_engine* e, float* crd, float* vel,
   };
   int rc = kOk;
   double best = 1e30, ms = 0.0;
-  int bu = e->pair_unroll, bb = e->pair_blocks_per_sm;
-  const bool rows = !(e->nl.clusters && !e->soft);
-  // candidates per lane per round and rows in flight per block (the row
-  // kernel of the plain single box) together, then blocks per SM
-  int bw = e->pair_warps;
-  const bool warps_knob = rows && !e->soft;
-  for (int u : {2, 4, 8})
-    for (int w : {4, 8, 16}) {
-      if (rc) break;
-      if (!rows && u != bu) continue;  // the cluster kernel has no unroll choice
-      if ((!warps_knob && w != bw) || (e->nsys > 0 && w == 4)) continue;
-      e->pair_unroll = u;
-      e->pair_warps = w;
-      e->pair_blocks_per_sm = 0;
-      if ((rc = measure_step(&ms))) break;  // the step, PME branch alongside
-      if (ms < best) {
-        best = ms;
-        bu = u;
-        bw = w;
-      }
-    }
-  e->pair_unroll = bu;
-  e->pair_warps = bw;
-  bb = 0;  // the joint search above ran at the occupancy maximum
-  for (int b : {2, 3}) {
-    if (rc) break;
+  // persistent blocks per SM of the pair kernel
+  int bb = 0;
+  for (int b : {0, 2, 3}) {
     e->pair_blocks_per_sm = b;
     if ((rc = measure_step(&ms))) break;
     if (ms < best) {
@@ -2217,20 +2271,6 @@ extern "C" int snb_engine_autotune(snb_engine* e, float* crd, float* vel,
     }
   }
   e->pair_blocks_per_sm = bb;
-  // the hit stash (phase 2 without gathers), same kernel otherwise
-  bool bst = e->pair_stash;
-  if (!rc && rows && !e->soft && e->nsys == 0) {
-    best = 1e30;
-    for (bool sx : {false, true}) {
-      e->pair_stash = sx;
-      if ((rc = measure_step(&ms))) break;
-      if (ms < best) {
-        best = ms;
-        bst = sx;
-      }
-    }
-  }
-  e->pair_stash = bst;
   int bs = e->nl.search_blocks_per_sm;
   best = 1e30;
   for (int b : {4, 8, 16}) {
@@ -2419,8 +2459,11 @@ extern "C" int snb_engine_set_list_form(snb_engine* e, int clusters) {
   if (!e) return fail(kBadInput, "engine_set_list_form: null handle");
   if (clusters && e->soft)
     return fail(kNotSupported, "engine_set_list_form: the soft-core kernel reads rows");
-  int rc = nl_set_clusters(e->nl, clusters != 0);
-  if (rc) return rc;
+  if (clusters && (e->nsys > 0 || !e->nl.trim))
+    return fail(kNotSupported,
+                "neighbor list: the cluster form needs one rectangular box of at least "
+                "five cells per axis");
+  e->cluster_form = clusters != 0;
   if (e->graph_exec) {  // the captured step holds the previous list form
     cudaGraphExecDestroy(e->graph_exec);
     cudaGraphDestroy(e->graph);
@@ -2469,21 +2512,13 @@ extern "C" int snb_engine_prune_passes(snb_engine* e, int* passes, long long* ke
   cudaStream_t st = S(stream);
   SNB_CUDA_TRY(cudaMemcpyAsync(passes, e->d_prune + 3, sizeof(int), cudaMemcpyDeviceToHost,
                                st));
-  std::vector<int> kept;
-  if (kept_entries) {
-    kept.resize(e->n);
-    SNB_CUDA_TRY(cudaMemcpyAsync(kept.data(), e->nl.d_row_in_count, sizeof(int) * e->n,
-                                 cudaMemcpyDeviceToHost, st));
-  }
   SNB_CUDA_TRY(cudaStreamSynchronize(st));
-  if (kept_entries)
-    for (int c : kept) *kept_entries += c;
-  return kOk;
+  return kept_entries ? nl_kept_entries(e->nl, kept_entries, st) : kOk;
 }
 
 extern "C" int snb_engine_list_form(snb_engine* e, int* clusters) {
   if (!e || !clusters) return fail(kBadInput, "engine_list_form: null argument");
-  *clusters = e->nl.clusters && !e->soft ? 1 : 0;
+  *clusters = e->cluster_form ? 1 : 0;
   return kOk;
 }
 
@@ -2548,6 +2583,11 @@ extern "C" int snb_engine_destroy(snb_engine* e) {
   cudaFree(e->d_cell_sys);
   cudaFree(e->d_box_need);
   cudaFree(e->d_prune);
+  cudaFree(e->d_lj_tab);
+  cudaFree(e->d_gtype);
+  cudaFree(e->d_soft_a);
+  cudaFree(e->d_soft_b);
+  cudaFree(e->d_soft_type);
   for (void* p : {(void*)e->d_ba, (void*)e->d_bb, (void*)e->d_bk, (void*)e->d_br0,
                   (void*)e->d_aa, (void*)e->d_ab, (void*)e->d_ac, (void*)e->d_ak,
                   (void*)e->d_at0})

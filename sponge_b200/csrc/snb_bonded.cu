@@ -33,9 +33,9 @@ __device__ __forceinline__ void bonded_virial(Accumulators& acc, int s, float3 f
 
 __device__ __forceinline__ void bonded_force(Accumulators& acc, int s, float3 f) {
   const int N = acc.n;
-  red_add(acc.d_f + s, to_fixed_force(f.x));
-  red_add(acc.d_f + N + s, to_fixed_force(f.y));
-  red_add(acc.d_f + 2 * N + s, to_fixed_force(f.z));
+  red_add(acc.d_f + s * acc.fs, to_fixed_force(f.x));
+  red_add(acc.d_f + s * acc.fs + acc.fc, to_fixed_force(f.y));
+  red_add(acc.d_f + s * acc.fs + 2 * acc.fc, to_fixed_force(f.z));
 }
 
 template <bool ENERGY, bool VIRIAL>

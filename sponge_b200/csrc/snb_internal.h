@@ -152,12 +152,7 @@ struct NeighborList {
   int* d_row_start = nullptr;   // [n + 1] = i * row_cap
   int* d_cols = nullptr;        // [n * row_cap] sorted-frame j of each pair
   int row_cap = 0;
-  // pruned rows (engine, single box): the entries of each row within
-  // cutoff + prune margin at the last prune pass, in the rows' layout, and
-  // the sorted positions that pass saw (null until nl_enable_prune)
-  int* d_cols_in = nullptr;     // [n * row_cap]
-  int* d_row_in_count = nullptr;  // [n]
-  float4* d_prune_ref = nullptr;  // [n]
+  float4* d_prune_ref = nullptr;  // [n] sorted positions the last prune pass saw
   long long cap = 0;
   int* d_unsorted = nullptr;    // [n] cell-binned caller indices before ordering
   int* d_sorted_cell = nullptr;  // [n] cell of each sorted atom
@@ -167,45 +162,41 @@ struct NeighborList {
   ScanScratch scan;
   long long last_total = 0;
   int generation = 0;
-  // Cluster form of the list (the engine's single-box step; needs at least
-  // five cells per axis).  Inside a cell the atoms follow a path up and down
-  // its four xy quarter columns, and every run of up to kClusterSize of them
-  // is one cluster.  Row c lists the j-clusters with a pair within r_l of
-  // i-cluster c: {first sorted atom of j, 4x4 pair mask | shift code << 16}.
-  // Pair-frame coordinates are crd - img_off (each atom in its build-time
-  // cell image); the shift code gives the periodic image of j's cell.
-  bool clusters = false;
-  int maxclus = 0;
+  // Grouped rows (the engine's list): a group is up to kGroupSize sorted
+  // atoms of one cell, whose atoms follow a path up and down the cell's four
+  // xy quarter columns.  Row g lists the partner atoms with a pair within r_l
+  // of group g as (sorted index << 8 | mask of the group's atoms), nearest
+  // first.  A cell's groups are numbered from cell_start / kGroupSize + cell,
+  // which leaves room for each cell's last, shorter group, so the numbers of
+  // a batch's systems do not depend on one another.  With groups the per-atom
+  // rows above are not allocated.
+  bool groups = false;
+  int max_groups = 0;
   int* d_atom_key = nullptr;     // [n] caller frame: order key inside the cell
-  int* d_clus_count = nullptr;   // [ncell] clusters of each cell
-  int* d_cell_clus = nullptr;    // [ncell + 1] first cluster of each cell
-  int2* d_clus = nullptr;        // [maxclus] {first sorted atom, atom count}
-  float4* d_clus_lo = nullptr;   // [maxclus] bounding box in the wrapped frame
-  float4* d_clus_hi = nullptr;
-  int* d_nclus = nullptr;        // [1] clusters of the last build
-  float3* d_img_off = nullptr;   // [n] sorted frame: box offset of the cell image
-  int* d_crow_count = nullptr;   // [maxclus]
-  int2* d_centry = nullptr;      // [maxclus * ccap]
-  int ccap = 0;
+  int2* d_group = nullptr;       // [max_groups] {first sorted atom, atom count}
+  int* d_grow_count = nullptr;   // [max_groups] entries of row g
+  int* d_gpairs = nullptr;       // [max_groups] pairs of row g
+  unsigned* d_gentry = nullptr;  // [max_groups * gcap]
+  unsigned char* d_gmask = nullptr;  // [max_groups * gcap / 32] (nl_enable_prune)
+  int gcap = 0;                  // a multiple of 32
 };
-constexpr int kClusterSize = 4;
-// Turns the cluster form on or off (single box, rectangular, at least five
-// cells per axis); the next update rebuilds.  Returns kNotSupported when the
-// box does not allow it.
-int nl_set_clusters(NeighborList& nl, bool on);
+constexpr int kGroupSize = 8;
+constexpr int kGroupMaxAtoms = 1 << 24;  // sorted indices that an entry holds
 
 int nl_init(NeighborList& nl, int n, float cutoff, float skin, const float* cell6,
             int refresh_interval, float skin_permit, int max_neighbor_numbers,
-            long long initial_capacity);
+            long long initial_capacity, bool groups = false);
 // A batch of rectangular boxes (sys[s].cell, rcell and atom ranges set);
 // fills the neighbor-grid fields of sys.  The caller sets nl.bv once the
 // SysGeom table is on the device.
 int nl_init_batch(NeighborList& nl, int n, float cutoff, float skin,
                   std::vector<SysGeom>& sys, int refresh_interval, float skin_permit,
-                  int max_neighbor_numbers);
+                  int max_neighbor_numbers, bool groups = false);
 void nl_free(NeighborList& nl);
-// Allocates the pruned rows (NeighborList::d_cols_in and the rest).
+// Allocates what the pruned rows need (the kept-atom bytes of grouped rows).
 int nl_enable_prune(NeighborList& nl);
+// Entries of the batches that the last prune pass kept (host sync).
+int nl_kept_entries(NeighborList& nl, long long* kept, cudaStream_t st);
 // Update as NEIGHBOR_LIST::Update (neighbor_list.cpp:974-1025): forced, or
 // conditional on the displacement check / refresh interval.  Device-side
 // decision; no host sync.
@@ -247,7 +238,13 @@ enum Accum { kAccumFixed = 0, kAccumFloat = 1 };
 // Per-atom accumulators in the sorted frame.
 struct Accumulators {
   int n = 0;
-  long long* d_f = nullptr;     // [3][n] fixed-point forces (2^40)
+  // fixed-point forces (2^40): component c of atom s at s * fs + c * fc.
+  // [3][n] for the modules, whose pair kernel adds runs of neighbouring
+  // atoms; [n][4] for the engine, where an atom's three components share one
+  // 32-byte sector.
+  long long* d_f = nullptr;
+  int fs = 1, fc = 0;
+  size_t f_len = 0;
   long long* d_e = nullptr;     // [n] fixed-point energy (2^32)  (pair owner)
   long long* d_elj = nullptr;   // [n] LJ part
   long long* d_ec = nullptr;    // [n] direct Coulomb part
@@ -258,7 +255,7 @@ struct Accumulators {
   long long* d_eaux = nullptr;  // [2][n] soft-core LJ energy inter / intra subsystem
   float* d_feaux = nullptr;     // [2][n] float version
 };
-int acc_init(Accumulators& a, int n);
+int acc_init(Accumulators& a, int n, bool by_atom = false);
 void acc_free(Accumulators& a);
 
 // ----------------------------------------------------------------------------
@@ -292,25 +289,12 @@ struct PairArgs {
   float cutoff2;
   float beta;
   BatchView bv;                 // nsys > 0: per-system boxes (rectangular)
-  int unroll = 4;               // scan candidates per lane per round (2, 4, 8)
-  int blocks_per_sm = 0;        // persistent blocks per SM, 0: occupancy maximum
-  int warps = 8;                // rows in flight per block (4, 8, 16)
-  bool stash = false;           // hits keep displacement / pair index (row kernel)
   // solvent split (single box): the atoms with global id >= solvent_begin
   // are the trailing water block.  solvent_mode 1: every pair but the
   // solvent-solvent ones (LENNARD_JONES_INFORMATION with solvent_numbers);
   // 2: only those (SOLVENT_LENNARD_JONES); 0: every pair
   int solvent_mode = 0;
   int solvent_begin = 0;
-  // pruned rows (solvent_mode 0; prune == null: full rows only).
-  // prune[0] != 0: a prune pass scans the full rows and keeps the entries
-  // within sqrt(prune2) in cols_in / row_in_count, with row i's position in
-  // prune_ref[i]; otherwise the scan reads cols_in / row_in_count.
-  const int* prune = nullptr;
-  int* cols_in = nullptr;
-  int* row_in_count = nullptr;
-  float4* prune_ref = nullptr;
-  float prune2 = 0.f;
 };
 int launch_pair(const PairArgs& a, Accumulators& acc, int accum, bool energy,
                 bool virial, bool ortho, cudaStream_t st);
@@ -328,27 +312,43 @@ int launch_prune_check(int n, const float3* crd, const int* map, const PruneChec
                        const Cell& cell, const Cell& rcell, cudaStream_t st,
                        const BatchView& bv);
 
-// The pair kernel over the cluster form of the list.
-struct ClusterPairArgs {
-  const int2* clus;             // {first sorted atom, atom count}
-  const int* nclus;             // device count of clusters
-  const int* crow_count;
-  const int2* centry;           // {first atom of j, mask | shift code << 16}
-  int ccap;
-  const float4* pos;            // pair frame (x,y,z,q), sorted
-  const int* type;              // sorted LJ type
-  const int* global;            // sorted -> global id (owner rule)
+// The engine's pair kernel over the grouped rows (plain LJ, or soft-core when
+// lj_b is given).  Atom types are packed: the type, with kTypeNoLJ when it has
+// no LJ against any type; for the soft-core kernel the A type in 15 bits, the
+// B type in the next 15, and the sign bit for an atom that may have a pair
+// whose end states differ.
+constexpr int kTypeNoLJ = 1 << 30;
+struct GroupArgs {
+  int n;
+  int ngroups;                  // group numbers in use (some hold no atoms)
+  const int2* group;
+  const int* row_count;
+  const unsigned* entry;
+  int cap;
+  const float4* pos;            // sorted (x,y,z,q)
+  const int* type;              // sorted packed types
   const int* nl_flags;          // skip when the list overflowed
-  const float* A;
-  const float* B;
+  const float2* lj;             // {A', B'} [n_types][n_types]
   int n_types;
-  float3 box;                   // rectangular box lengths (image shifts)
-  float cutoff2;
+  Cell cell, rcell;
+  float cutoff, cutoff2;
   float beta;
-  int blocks_per_sm = 0;        // persistent blocks per SM, 0: occupancy maximum
+  BatchView bv;
+  int split_log2 = 0;
+  int blocks_per_sm = 0;
+  // prune passes: prune[0] != 0 takes every batch and notes in mask the i
+  // atoms with a partner within sqrt(prune2), and the positions in prune_ref
+  const int* prune = nullptr;
+  unsigned char* mask = nullptr;
+  float4* prune_ref = nullptr;
+  float prune2 = 0.f, prune_r = 0.f;
+  // soft-core: state B table and parameters
+  const float2* lj_b = nullptr;
+  int n_types_b = 0;
+  float lambda = 0.f, alp_A = 0.f, alp_B = 0.f, sigma6 = 0.f, sigma6_min = 0.f;
 };
-int launch_pair_clusters(const ClusterPairArgs& a, Accumulators& acc, int accum,
-                         bool energy, bool virial, cudaStream_t st);
+int launch_pair_groups(GroupArgs a, Accumulators& acc, bool energy, bool virial,
+                       cudaStream_t st);
 
 // Rigid triangle: atoms A, B, C, canonical frame (A at (0, ra), B at (rc, rb),
 // C at (rd, re) about the centre of mass) and masses.
@@ -425,19 +425,9 @@ struct SoftArgs {
   float beta;
   float lambda, alpha, p;
   float sigma6, sigma6_min;
-  // pruned rows of the engine's row kernel, as PairArgs::prune
-  const int* prune = nullptr;
-  int* cols_in = nullptr;
-  int* row_in_count = nullptr;
-  float4* prune_ref = nullptr;
-  float prune2 = 0.f;
 };
 int launch_soft(const SoftArgs& a, Accumulators& acc, int accum, bool energy,
                 bool virial, bool dudl, long long* dudl_total, cudaStream_t st);
-// The engine's soft-core pair kernel (fixed point, rectangular box).
-int launch_soft_rows(const SoftArgs& a, Accumulators& acc, bool energy, bool virial,
-                     cudaStream_t st);
-
 // ----------------------------------------------------------------------------
 // One axis of the convolution's own FFT passes (snb_fft.cuh): length and
 // radices in stage order.
@@ -548,11 +538,8 @@ int fft_size(float length);
 int pme_reciprocal(PME& p, const float4* pos, int n, Accumulators& acc,
                    int accum, bool need_energy, bool need_virial,
                    cudaStream_t st);
-// img_off (may be null): sorted-frame offsets subtracted from the pair
-// frame's coordinates (pos) only; the PME binning takes crd as given.
 int pme_pack_bin(PME& p, int n, const float3* crd, const float* charge, const int* type,
-                 const int* perm, float4* pos, int* type_sorted, cudaStream_t st,
-                 const float3* img_off = nullptr);
+                 const int* perm, float4* pos, int* type_sorted, cudaStream_t st);
 int pme_after_bin(PME& p, int n, Accumulators& acc, int accum, bool need_energy,
                   bool need_virial, cudaStream_t st);
 // Virtual atoms for the engine: positions refreshed in crd (caller frame),
@@ -580,10 +567,9 @@ int launch_excluded(int n, const float3* crd, const float* charge,
 
 // ----------------------------------------------------------------------------
 // Frame conversion kernels.
-// pos[s] = (crd[perm[s]] - img_off[s] (when given), charge[perm[s]]).
+// pos[s] = (crd[perm[s]], charge[perm[s]]).
 int launch_pack(int n, const float3* crd, const float* charge, const int* type,
-                const int* perm, float4* pos, int* type_sorted, cudaStream_t st,
-                const float3* img_off = nullptr);
+                const int* perm, float4* pos, int* type_sorted, cudaStream_t st);
 // frc[caller i] += acc[map[i]] (converted), optional energies/virials, then
 // zero the accumulators.
 int launch_unpack(int n, const int* map, Accumulators& acc, int accum,

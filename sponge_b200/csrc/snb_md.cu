@@ -15,9 +15,9 @@ namespace snb {
 __device__ __forceinline__ void acc_force(Accumulators& acc, int s, float fx, float fy,
                                           float fz) {
   const int N = acc.n;
-  red_add(acc.d_f + s, to_fixed_force(fx));
-  red_add(acc.d_f + N + s, to_fixed_force(fy));
-  red_add(acc.d_f + 2 * N + s, to_fixed_force(fz));
+  red_add(acc.d_f + s * acc.fs, to_fixed_force(fx));
+  red_add(acc.d_f + s * acc.fs + acc.fc, to_fixed_force(fy));
+  red_add(acc.d_f + s * acc.fs + 2 * acc.fc, to_fixed_force(fz));
 }
 
 // Bonds and angles in one launch: the first ceil(nb/256) blocks take bonds.
@@ -125,9 +125,8 @@ __global__ void k_leap_frog(int n, const int* __restrict__ map, Accumulators acc
   float3 r = crd[i];
   float3 r_old = make_float3(0.f, 0.f, 0.f);
   if (old_crd) r_old = old_crd[i];
-  const int N = acc.n;
-  const long long* __restrict__ f = acc.d_f;
-  const long long fx_i = f[s], fy_i = f[N + s], fz_i = f[2 * N + s];
+  const long long* __restrict__ f = acc.d_f + s * acc.fs;
+  const long long fx_i = f[0], fy_i = f[acc.fc], fz_i = f[2 * acc.fc];
   const float fx = (float)((double)fx_i * kForceScaleInv);
   const float fy = (float)((double)fy_i * kForceScaleInv);
   const float fz = (float)((double)fz_i * kForceScaleInv);
@@ -204,7 +203,7 @@ int launch_leap_frog(int n, const int* map, Accumulators& acc, float3* crd,
   SNB_CUDA_TRY(cudaGetLastError());
   // the accumulator starts the next step at zero: one coalesced clear
   // instead of scattered stores through the permutation
-  SNB_CUDA_TRY(cudaMemsetAsync(acc.d_f, 0, sizeof(long long) * 3 * (size_t)acc.n, st));
+  SNB_CUDA_TRY(cudaMemsetAsync(acc.d_f, 0, sizeof(long long) * acc.f_len, st));
   return kOk;
 }
 

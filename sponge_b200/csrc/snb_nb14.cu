@@ -36,12 +36,12 @@ __global__ void k_nb14(int m, const int* __restrict__ ia, const int* __restrict_
   const float fs = -A[t] * ir14 + B[t] * ir8 - cf[t] * ir2 * ir * qa * qb;
   const float gx = fs * d.x, gy = fs * d.y, gz = fs * d.z;
   const int N = acc.n;
-  red_add(acc.d_f + a, to_fixed_force(gx));
-  red_add(acc.d_f + N + a, to_fixed_force(gy));
-  red_add(acc.d_f + 2 * N + a, to_fixed_force(gz));
-  red_add(acc.d_f + b, to_fixed_force(-gx));
-  red_add(acc.d_f + N + b, to_fixed_force(-gy));
-  red_add(acc.d_f + 2 * N + b, to_fixed_force(-gz));
+  red_add(acc.d_f + a * acc.fs, to_fixed_force(gx));
+  red_add(acc.d_f + a * acc.fs + acc.fc, to_fixed_force(gy));
+  red_add(acc.d_f + a * acc.fs + 2 * acc.fc, to_fixed_force(gz));
+  red_add(acc.d_f + b * acc.fs, to_fixed_force(-gx));
+  red_add(acc.d_f + b * acc.fs + acc.fc, to_fixed_force(-gy));
+  red_add(acc.d_f + b * acc.fs + 2 * acc.fc, to_fixed_force(-gz));
   if (ENERGY) {
     const float ec = cf[t] * ir * qa * qb;
     // the reference's constants 0.08333333 and 0.1666666 (nb14.cpp:83-85)

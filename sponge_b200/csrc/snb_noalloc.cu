@@ -105,6 +105,8 @@ extern "C" int snb_pme_excluded_force_noalloc(
   Accumulators acc;
   acc.n = atom_numbers;
   acc.d_f = scratch;
+  acc.fs = 1;
+  acc.fc = atom_numbers;
   acc.d_e = scratch + 3 * n;
   acc.d_elj = acc.d_e + n;
   acc.d_ec = acc.d_e + 2 * n;

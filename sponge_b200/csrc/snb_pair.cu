@@ -36,9 +36,9 @@ __device__ __forceinline__ void add_force(Accumulators& acc, int s, float fx,
                                           float fy, float fz) {
   const int N = acc.n;
   if (ACCUM == kAccumFixed) {
-    red_add(acc.d_f + s, to_fixed_force(fx));
-    red_add(acc.d_f + N + s, to_fixed_force(fy));
-    red_add(acc.d_f + 2 * N + s, to_fixed_force(fz));
+    red_add(acc.d_f + s * acc.fs, to_fixed_force(fx));
+    red_add(acc.d_f + s * acc.fs + acc.fc, to_fixed_force(fy));
+    red_add(acc.d_f + s * acc.fs + 2 * acc.fc, to_fixed_force(fz));
   } else {
     atomicAdd(acc.d_ff + s, fx);
     atomicAdd(acc.d_ff + N + s, fy);
@@ -82,14 +82,7 @@ __device__ __forceinline__ void add_virial(Accumulators& acc, int s, const float
 // holds is taken in several rounds.
 constexpr int kWarps = 8;      // rows in flight per block (warps per block)
 constexpr int kHitCap = 512;   // per-warp hit list (entries)
-// STASH: phase 1 keeps, per hit, the displacement and charge (float4) and
-// the atom and LJ type-pair index (int2) in dynamic shared memory, so that
-// phase 2 gathers nothing from global memory; the displacement is the one
-// the cutoff test used, so the results are bitwise those of the plain list.
-constexpr int kStashCap = 256;
-// candidates per lane per scan round: a template parameter (2, 4 or 8), and
-// rows in flight per block (4, 8 or 16 warps), that the engine's autotuner
-// picks; 4 and 8 elsewhere
+constexpr int kScanU = 4;      // candidates per lane per scan round
 
 // The pair terms of i and j with the LJ coefficients A' = 12 A, B' = 6 B of
 // their type pair.  COUL_ONLY: atom i's type has A' = B' = 0 with every
@@ -166,20 +159,14 @@ __device__ __forceinline__ void lj_pair(const Args& a, Accumulators& acc,
 
 // SOLV 1 / 2: the solvent split of PairArgs::solvent_mode (pairs with both
 // global ids >= solvent_begin left out / taken alone); 0: every pair.
-template <int ACCUM, bool ENERGY, bool VIRIAL, bool ORTHO, bool BATCH, int kScanU,
-          int SOLV = 0, int WARPS = kWarps, bool STASH = false>
-__global__ void __launch_bounds__(32 * WARPS, 32 / WARPS)
+template <int ACCUM, bool ENERGY, bool VIRIAL, bool ORTHO, bool BATCH, int SOLV = 0>
+__global__ void __launch_bounds__(32 * kWarps, 32 / kWarps)
 k_lj_direct(PairArgs a, Accumulators acc) {
-  constexpr int kCap = STASH ? kStashCap : kHitCap;
-  static_assert(kScanU >= 1 && 32 * kScanU < kCap, "scan round exceeds the hit list");
-  extern __shared__ float4 sh_dyn[];
-  __shared__ int hits_all[STASH ? 1 : WARPS][STASH ? 1 : kHitCap];
+  static_assert(32 * kScanU < kHitCap, "scan round exceeds the hit list");
+  extern __shared__ float sh_dyn[];
+  __shared__ int hits_all[kWarps][kHitCap];
   const int npair = a.n_types * (a.n_types + 1) / 2;
-  // dynamic shared memory: [stash e: WARPS][kCap] float4, [stash jt] int2,
-  // then the LJ tables
-  float4* stash_e = sh_dyn;
-  int2* stash_jt = reinterpret_cast<int2*>(sh_dyn + (STASH ? WARPS * kCap : 0));
-  float* sA = reinterpret_cast<float*>(stash_jt + (STASH ? WARPS * kCap : 0));
+  float* sA = sh_dyn;
   float* sB = sA + npair;
   for (int k = threadIdx.x; k < npair; k += blockDim.x) {
     sA[k] = a.A[k];
@@ -188,24 +175,17 @@ k_lj_direct(PairArgs a, Accumulators acc) {
   __syncthreads();
   const int lane = threadIdx.x & 31;
   const int w = threadIdx.x >> 5;
-  int* hits = hits_all[STASH ? 0 : w];
-  float4* se = stash_e + (STASH ? w * kCap : 0);
-  int2* sjt = stash_jt + (STASH ? w * kCap : 0);
+  int* hits = hits_all[w];
   if (a.nl_flags && a.nl_flags[1]) return;  // list overflowed: rows not written
-  // Pruned rows: a prune pass scans the full rows and keeps the candidates
-  // within cutoff + margin; the steps between scan only those.
-  constexpr bool kPrunable = SOLV == 0;
-  const bool prune_pass = kPrunable && a.prune != nullptr && a.prune[0] != 0;
-  const bool use_inner = kPrunable && a.prune != nullptr && !prune_pass;
-  const int* __restrict__ cols = use_inner ? a.cols_in : a.cols;
-  const int* __restrict__ rcount = use_inner ? a.row_in_count : a.row_count;
+  const int* __restrict__ cols = a.cols;
+  const int* __restrict__ rcount = a.row_count;
   // Each block owns a contiguous range of sorted atoms, so the neighbours its
   // warps gather overlap and stay in this SM's L1.
   const int per_block = (a.n + gridDim.x - 1) / gridDim.x;
   const int i_begin = blockIdx.x * per_block;
   const int i_end = min(a.n, i_begin + per_block);
   const unsigned lt = (1u << lane) - 1u;
-  for (int i = i_begin + w; i < i_end; i += WARPS) {
+  for (int i = i_begin + w; i < i_end; i += kWarps) {
   const float4 pi = a.pos[i];
   const float3 ri = make_float3(pi.x, pi.y, pi.z);
   const int ti = a.type[i];
@@ -219,7 +199,6 @@ k_lj_direct(PairArgs a, Accumulators acc) {
   float e_lj = 0.f, e_c = 0.f;
   float vir[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
   const int k0 = a.row_start[i], k1 = k0 + rcount[i];
-  int kept = 0;  // prune pass: entries kept so far
   // a type without LJ against every type (water H): Coulomb-only row
   bool coul_only = true;
   for (int t = lane; t < a.n_types; t += 32) {
@@ -230,7 +209,7 @@ k_lj_direct(PairArgs a, Accumulators acc) {
   {
     // the warp's next row: start pulling its indices from HBM into L2 now
     // (row starts are multiples of 8 entries, so 16-byte aligned)
-    const int inext = i + WARPS;
+    const int inext = i + kWarps;
     if (lane == 0 && inext < i_end) {
       const int cn = rcount[inext];
       if (cn > 0)
@@ -239,92 +218,53 @@ k_lj_direct(PairArgs a, Accumulators acc) {
   }
   // hits of the row taken in earlier rounds: lane l takes the row's hits
   // l, l + 32, ... in order whatever the rounds, so the float sums of i's
-  // force are the same for every hit-list capacity and scan width
+  // force do not depend on how the rounds fall
   int done = 0;
-  // with up to 4 candidates per lane, each round's indices are loaded one
-  // round ahead, so the gathers of a round wait only on their own load (at 8
-  // the extra registers spill).  The index stream is read once: loaded
-  // evict-first (__ldcs) so that L1 keeps the positions the rows share.
-  constexpr bool kAhead = kScanU <= 4;
+  // each round's indices are loaded one round ahead, so the gathers of a
+  // round wait only on their own load.  The index stream is read once:
+  // loaded evict-first (__ldcs) so that L1 keeps the positions the rows share.
   int jn[kScanU];
 #pragma unroll
   for (int u = 0; u < kScanU; ++u) {
     const int k = k0 + 32 * u + lane;
-    jn[u] = kAhead && k < k1 ? __ldcs(cols + k) : -1;
+    jn[u] = k < k1 ? __ldcs(cols + k) : -1;
   }
   for (int base = k0; base < k1;) {
     // phase 1: candidates -> hit list
     int count = 0;
-    for (; base < k1 && count <= kCap - 32 * kScanU; base += 32 * kScanU) {
+    for (; base < k1 && count <= kHitCap - 32 * kScanU; base += 32 * kScanU) {
       int jj[kScanU];
 #pragma unroll
       for (int u = 0; u < kScanU; ++u) {
-        if (kAhead) {
-          jj[u] = jn[u];
-          const int k = base + 32 * (kScanU + u) + lane;
-          jn[u] = k < k1 ? __ldcs(cols + k) : -1;
-        } else {
-          const int k = base + 32 * u + lane;
-          jj[u] = k < k1 ? __ldcs(cols + k) : -1;
-        }
+        jj[u] = jn[u];
+        const int k = base + 32 * (kScanU + u) + lane;
+        jn[u] = k < k1 ? __ldcs(cols + k) : -1;
       }
       float4 pp[kScanU];
-      int tt[kScanU];
 #pragma unroll
-      for (int u = 0; u < kScanU; ++u) {
+      for (int u = 0; u < kScanU; ++u)
         if (jj[u] >= 0) pp[u] = a.pos[jj[u]];
-        tt[u] = STASH && !coul_only && jj[u] >= 0 ? a.type[jj[u]] : 0;
-      }
 #pragma unroll
       for (int u = 0; u < kScanU; ++u) {
-        bool in = false, keep = false;
+        bool in = false;
         if (jj[u] >= 0) {
           const float3 dr = min_image_fast<ORTHO>(make_float3(pp[u].x, pp[u].y, pp[u].z),
                                                   ri, cell, rcell);
-          const float d2 = dr.x * dr.x + dr.y * dr.y + dr.z * dr.z;
-          in = d2 < a.cutoff2;
-          keep = kPrunable && d2 < a.prune2;
+          in = dr.x * dr.x + dr.y * dr.y + dr.z * dr.z < a.cutoff2;
           if (SOLV && in) {
             const bool both = i_solvent && a.global[jj[u]] >= a.solvent_begin;
             in = SOLV == 1 ? !both : both;
           }
         }
-        if (kPrunable && prune_pass) {  // warp-uniform
-          const unsigned mk = __ballot_sync(0xffffffffu, keep);
-          if (keep) a.cols_in[k0 + kept + __popc(mk & lt)] = jj[u];
-          kept += __popc(mk);
-        }
         const unsigned m = __ballot_sync(0xffffffffu, in);
-        if (in) {
-          const int slot = count + __popc(m & lt);
-          if (STASH) {
-            const float3 dr = min_image_fast<ORTHO>(make_float3(pp[u].x, pp[u].y, pp[u].z),
-                                                    ri, cell, rcell);
-            se[slot] = make_float4(dr.x, dr.y, dr.z, pp[u].w);
-            sjt[slot] = make_int2(jj[u], coul_only ? 0 : lj_pair_index(ti, tt[u]));
-          } else {
-            hits[slot] = jj[u];
-          }
-        }
+        if (in) hits[count + __popc(m & lt)] = jj[u];
         count += __popc(m);
       }
     }
     __syncwarp();
     // phase 2: pair terms over the hit list
     const int h0 = (lane - done) & 31;
-    if (STASH && coul_only) {
-      for (int h = h0; h < count; h += 32) {
-        const int2 jt = sjt[h];
-        lj_pair_ab<ACCUM, ENERGY, VIRIAL, true>(a, acc, 0.f, 0.f, pi.w, gi, se[h], jt.x, fx,
-                                                fy, fz, e_lj, e_c, vir);
-      }
-    } else if (STASH) {
-      for (int h = h0; h < count; h += 32) {
-        const int2 jt = sjt[h];
-        lj_pair_ab<ACCUM, ENERGY, VIRIAL>(a, acc, sA[jt.y], sB[jt.y], pi.w, gi, se[h], jt.x,
-                                          fx, fy, fz, e_lj, e_c, vir);
-      }
-    } else if (coul_only) {
+    if (coul_only) {
       for (int h = h0; h < count; h += 32) {
         const int j = hits[h];
         const float4 pj = a.pos[j];
@@ -349,10 +289,6 @@ k_lj_direct(PairArgs a, Accumulators acc) {
     done += count;
     __syncwarp();
   }
-  if (kPrunable && prune_pass && lane == 0) {
-    a.row_in_count[i] = kept;
-    a.prune_ref[i] = pi;
-  }
   fx = warp_sum(fx);
   fy = warp_sum(fy);
   fz = warp_sum(fz);
@@ -374,19 +310,6 @@ k_lj_direct(PairArgs a, Accumulators acc) {
 
 using RowKern = void (*)(PairArgs, Accumulators);
 
-// The plain single-box row kernel of W warps per block with or without the
-// hit stash (which needs at most 4 candidates per lane per round).
-template <int ACCUM, bool ENERGY, bool VIRIAL, int W, bool S>
-static RowKern row_kernel(int u) {
-  if constexpr (S)
-    return u == 2 ? k_lj_direct<ACCUM, ENERGY, VIRIAL, true, false, 2, 0, W, true>
-                  : k_lj_direct<ACCUM, ENERGY, VIRIAL, true, false, 4, 0, W, true>;
-  else
-    return u == 2 ? k_lj_direct<ACCUM, ENERGY, VIRIAL, true, false, 2, 0, W>
-         : u == 8 ? k_lj_direct<ACCUM, ENERGY, VIRIAL, true, false, 8, 0, W>
-                  : k_lj_direct<ACCUM, ENERGY, VIRIAL, true, false, 4, 0, W>;
-}
-
 // Raises a kernel's dynamic shared memory limit once, when it needs more
 // than the default 48 KB.
 static void allow_smem(RowKern k, size_t smem) {
@@ -402,63 +325,27 @@ static void allow_smem(RowKern k, size_t smem) {
 
 template <int ACCUM, bool ENERGY, bool VIRIAL>
 static void launch3(const PairArgs& a, Accumulators& acc, bool ortho, cudaStream_t st) {
-  size_t smem = sizeof(float) * a.n_types * (a.n_types + 1);
+  const size_t smem = sizeof(float) * a.n_types * (a.n_types + 1);
   RowKern kern;
-  // the launch-shape choices apply to the MD step's variant (fixed point,
-  // force only, rectangular, one box, no solvent split); the others take 4
-  // candidates per lane and 8 warps without the stash
-  constexpr bool kTunable = ACCUM == kAccumFixed && !ENERGY && !VIRIAL;
-  const bool tunable = kTunable && ortho;
-  const bool single = a.bv.nsys == 0 && a.solvent_mode == 0;
-  const int u = tunable ? a.unroll : 4;
-  // rows in flight per block: 4, 8 or 16 warps for one box, 8 or 16 for a
-  // batch; 8 for the other variants
-  int wb = kWarps;
-  if (tunable && a.solvent_mode == 0)
-    wb = a.bv.nsys == 0 ? a.warps : (a.warps == 16 ? 16 : kWarps);
-  const bool stash = tunable && single && a.stash;
   if (a.solvent_mode != 0 && a.bv.nsys == 0)
-    kern = ortho ? (a.solvent_mode == 1 ? k_lj_direct<ACCUM, ENERGY, VIRIAL, true, false, 4, 1>
-                                        : k_lj_direct<ACCUM, ENERGY, VIRIAL, true, false, 4, 2>)
-                 : (a.solvent_mode == 1 ? k_lj_direct<ACCUM, ENERGY, VIRIAL, false, false, 4, 1>
-                                        : k_lj_direct<ACCUM, ENERGY, VIRIAL, false, false, 4, 2>);
-  else if (a.bv.nsys > 0 && kTunable && wb == 16)
-    kern = u == 2 ? k_lj_direct<ACCUM, ENERGY, VIRIAL, true, true, 2, 0, 16>
-         : u == 8 ? k_lj_direct<ACCUM, ENERGY, VIRIAL, true, true, 8, 0, 16>
-                  : k_lj_direct<ACCUM, ENERGY, VIRIAL, true, true, 4, 0, 16>;
+    kern = ortho ? (a.solvent_mode == 1 ? k_lj_direct<ACCUM, ENERGY, VIRIAL, true, false, 1>
+                                        : k_lj_direct<ACCUM, ENERGY, VIRIAL, true, false, 2>)
+                 : (a.solvent_mode == 1 ? k_lj_direct<ACCUM, ENERGY, VIRIAL, false, false, 1>
+                                        : k_lj_direct<ACCUM, ENERGY, VIRIAL, false, false, 2>);
   else if (a.bv.nsys > 0)
-    kern = u == 2 ? k_lj_direct<ACCUM, ENERGY, VIRIAL, true, true, 2>
-         : u == 8 ? k_lj_direct<ACCUM, ENERGY, VIRIAL, true, true, 8>
-                  : k_lj_direct<ACCUM, ENERGY, VIRIAL, true, true, 4>;
-  else if (ortho) {
-    if constexpr (kTunable) {
-      if (wb == 4)
-        kern = stash ? row_kernel<ACCUM, ENERGY, VIRIAL, 4, true>(u)
-                     : row_kernel<ACCUM, ENERGY, VIRIAL, 4, false>(u);
-      else if (wb == 16)
-        kern = stash ? row_kernel<ACCUM, ENERGY, VIRIAL, 16, true>(u)
-                     : row_kernel<ACCUM, ENERGY, VIRIAL, 16, false>(u);
-      else
-        kern = stash ? row_kernel<ACCUM, ENERGY, VIRIAL, kWarps, true>(u)
-                     : row_kernel<ACCUM, ENERGY, VIRIAL, kWarps, false>(u);
-    } else {
-      kern = row_kernel<ACCUM, ENERGY, VIRIAL, kWarps, false>(u);
-    }
-  } else {
-    kern = k_lj_direct<ACCUM, ENERGY, VIRIAL, false, false, 4>;
-  }
-  if (stash) smem += (sizeof(float4) + sizeof(int2)) * (size_t)wb * kStashCap;
+    kern = k_lj_direct<ACCUM, ENERGY, VIRIAL, true, true>;
+  else
+    kern = ortho ? k_lj_direct<ACCUM, ENERGY, VIRIAL, true, false>
+                 : k_lj_direct<ACCUM, ENERGY, VIRIAL, false, false>;
   allow_smem(kern, smem);
-  // persistent grid: as many blocks as fit at once, or the tuned count
+  // persistent grid: as many blocks as fit at once
   static int sms = 0;
   if (!sms) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, 0);
-  const int threads = 32 * wb;
   int per_sm = 1;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32 * kWarps, smem);
   per_sm = std::max(per_sm, 1);
-  if (a.blocks_per_sm > 0) per_sm = std::min(per_sm, a.blocks_per_sm);
-  int blocks = std::max(1, std::min(sms * per_sm, ceil_div(a.n, threads / 32)));
-  kern<<<blocks, threads, smem, st>>>(a, acc);
+  const int blocks = std::max(1, std::min(sms * per_sm, ceil_div(a.n, kWarps)));
+  kern<<<blocks, 32 * kWarps, smem, st>>>(a, acc);
 }
 
 template <int ACCUM>
@@ -483,221 +370,6 @@ int launch_pair(const PairArgs& a, Accumulators& acc, int accum, bool energy,
     launch2<kAccumFloat>(a, acc, energy, virial, ortho, st);
   SNB_CUDA_TRY(cudaGetLastError());
   return kOk;
-}
-
-// ---------------------------------------------------------------------------
-// The same pair terms over the cluster form of the list.  One warp per
-// i-cluster (up to four sorted atoms, held in every lane's registers) at a
-// time.  Phase 1 scans the row eight entries per round: lane l takes entry
-// l/4 and its j atom l%4 (one 16-byte load, the entry's periodic image
-// added), tests it against the four i atoms under the entry's mask and the
-// cutoff, and appends each hit to the list of its i atom (ballot + popc):
-// no index load per candidate, and the j atoms of an entry are contiguous.
-// Phase 2 runs the pair terms of each i atom's list 32 at a time as the row
-// kernel does, i force in registers, j forces to the accumulators.
-// Coordinates are in the pair frame (each atom in its cell's image), so the
-// displacement is (x_j + shift) - x_i with no rounding to an image.
-constexpr int kCWarps = 8;
-constexpr int kSubCap = 256;  // per i atom list of hits
-constexpr int kCScanU = 2;    // rounds of eight entries in flight in phase 1
-
-template <int ACCUM, bool ENERGY, bool VIRIAL>
-__global__ void __launch_bounds__(32 * kCWarps, 3)
-k_lj_clusters(ClusterPairArgs a, Accumulators acc) {
-  extern __shared__ float sh_tab[];
-  __shared__ int hits_all[kCWarps][kClusterSize][kSubCap];
-  __shared__ float4 shift_tab[27];
-  float* sA = sh_tab;
-  float* sB = sh_tab + a.n_types * (a.n_types + 1) / 2;
-  const int npair = a.n_types * (a.n_types + 1) / 2;
-  for (int k = threadIdx.x; k < npair; k += blockDim.x) {
-    sA[k] = a.A[k];
-    sB[k] = a.B[k];
-  }
-  if (threadIdx.x < 27) {
-    const int k = threadIdx.x;
-    shift_tab[k] = make_float4((float)(k / 9 - 1) * a.box.x, (float)((k / 3) % 3 - 1) * a.box.y,
-                               (float)(k % 3 - 1) * a.box.z, 0.f);
-  }
-  __syncthreads();
-  if (a.nl_flags && a.nl_flags[1]) return;  // list overflowed: rows not written
-  const int lane = threadIdx.x & 31;
-  const int w = threadIdx.x >> 5;
-  const unsigned lt = (1u << lane) - 1u;
-  const int nclus = *a.nclus;
-  const int per_block = (nclus + gridDim.x - 1) / gridDim.x;
-  const int c_end = min(nclus, (int)blockIdx.x * per_block + per_block);
-  for (int c = blockIdx.x * per_block + w; c < c_end; c += kCWarps) {
-    const int2 ci = a.clus[c];
-    // the i atoms, broadcast from lanes 0..3
-    const bool own = lane < ci.y;
-    const float4 pl = own ? a.pos[ci.x + lane] : make_float4(0.f, 0.f, 0.f, 0.f);
-    const int tl = own ? a.type[ci.x + lane] : 0;
-    const int gl = (ENERGY || VIRIAL) && own ? a.global[ci.x + lane] : 0;
-    float4 p_i[kClusterSize];
-    int t_i[kClusterSize], g_i[kClusterSize];
-    bool coul_only[kClusterSize];
-#pragma unroll
-    for (int ii = 0; ii < kClusterSize; ++ii) {
-      p_i[ii] = make_float4(__shfl_sync(0xffffffffu, pl.x, ii), __shfl_sync(0xffffffffu, pl.y, ii),
-                            __shfl_sync(0xffffffffu, pl.z, ii), __shfl_sync(0xffffffffu, pl.w, ii));
-      t_i[ii] = __shfl_sync(0xffffffffu, tl, ii);
-      g_i[ii] = __shfl_sync(0xffffffffu, gl, ii);
-      // a type without LJ against every type (water H): Coulomb-only terms
-      bool co = true;
-      for (int t = lane; t < a.n_types; t += 32) {
-        const int p = lj_pair_index(t_i[ii], t);
-        co = co && sA[p] == 0.f && sB[p] == 0.f;
-      }
-      coul_only[ii] = __all_sync(0xffffffffu, co);
-    }
-    float f_i[kClusterSize][3];
-    float elj_i[kClusterSize], ec_i[kClusterSize], vir_i[kClusterSize][6];
-#pragma unroll
-    for (int ii = 0; ii < kClusterSize; ++ii) {
-      f_i[ii][0] = f_i[ii][1] = f_i[ii][2] = 0.f;
-      elj_i[ii] = ec_i[ii] = 0.f;
-#pragma unroll
-      for (int q = 0; q < 6; ++q) vir_i[ii][q] = 0.f;
-    }
-    const int n_ent = min(a.crow_count[c], a.ccap);
-    const int2* row = a.centry + (size_t)c * a.ccap;
-    {
-      // the warp's next row: start pulling its entries into L2 now (rows
-      // start on 32-byte boundaries)
-      const int cn = c + kCWarps;
-      if (lane == 0 && cn < c_end) {
-        const int m = min(a.crow_count[cn], a.ccap);
-        if (m > 0)
-          prefetch_l2(a.centry + (size_t)cn * a.ccap, (unsigned)(m * 8 + 15) & ~15u);
-      }
-    }
-    const int jl = lane & 3, eo = lane >> 2;
-    for (int base = 0; base < n_ent;) {
-      // phase 1: candidates -> per-i hit lists, kCScanU rounds of eight
-      // entries in flight per pass
-      int cnt[kClusterSize] = {0, 0, 0, 0};
-      for (; base < n_ent &&
-             max(max(cnt[0], cnt[1]), max(cnt[2], cnt[3])) <= kSubCap - 32 * kCScanU;
-           base += 8 * kCScanU) {
-        int2 en[kCScanU];
-#pragma unroll
-        for (int u = 0; u < kCScanU; ++u) {
-          const int e = base + 8 * u + eo;
-          en[u] = e < n_ent ? row[e] : make_int2(0, 0);
-        }
-        float4 pp[kCScanU];
-#pragma unroll
-        for (int u = 0; u < kCScanU; ++u)
-          if (((unsigned)en[u].y >> jl) & 0x1111u) pp[u] = a.pos[en[u].x + jl];
-#pragma unroll
-        for (int u = 0; u < kCScanU; ++u) {
-          const unsigned col = ((unsigned)en[u].y >> jl) & 0x1111u;
-          const unsigned code = ((unsigned)en[u].y >> 16) & 31u;
-          float3 pj = make_float3(0.f, 0.f, 0.f);
-          if (col) {
-            const float4 sh = shift_tab[code];
-            pj = make_float3(pp[u].x + sh.x, pp[u].y + sh.y, pp[u].z + sh.z);
-          }
-          const int hcode = (en[u].x + jl) | (int)(code << 27);
-#pragma unroll
-          for (int ii = 0; ii < kClusterSize; ++ii) {
-            bool hit = false;
-            if ((col >> (4 * ii)) & 1u) {
-              const float dx = pj.x - p_i[ii].x, dy = pj.y - p_i[ii].y, dz = pj.z - p_i[ii].z;
-              hit = dx * dx + dy * dy + dz * dz < a.cutoff2;
-            }
-            const unsigned m = __ballot_sync(0xffffffffu, hit);
-            if (hit) hits_all[w][ii][cnt[ii] + __popc(m & lt)] = hcode;
-            cnt[ii] += __popc(m);
-          }
-        }
-      }
-      __syncwarp();
-      // phase 2: pair terms of each i atom's hits
-#pragma unroll
-      for (int ii = 0; ii < kClusterSize; ++ii) {
-        const int* hits = hits_all[w][ii];
-        if (coul_only[ii]) {
-          for (int h = lane; h < cnt[ii]; h += 32) {
-            const int hc = hits[h];
-            const int jj = hc & 0x7FFFFFF;
-            const float4 pj = a.pos[jj];
-            const float4 sh = shift_tab[(unsigned)hc >> 27];
-            lj_pair<ACCUM, ENERGY, VIRIAL, true>(
-                a, acc, sA, sB, t_i[ii], p_i[ii].w, g_i[ii],
-                make_float4(pj.x + sh.x - p_i[ii].x, pj.y + sh.y - p_i[ii].y,
-                            pj.z + sh.z - p_i[ii].z, pj.w),
-                jj, 0, f_i[ii][0], f_i[ii][1], f_i[ii][2], elj_i[ii], ec_i[ii], vir_i[ii]);
-          }
-        } else {
-          for (int h = lane; h < cnt[ii]; h += 32) {
-            const int hc = hits[h];
-            const int jj = hc & 0x7FFFFFF;
-            const float4 pj = a.pos[jj];
-            const int tj = a.type[jj];
-            const float4 sh = shift_tab[(unsigned)hc >> 27];
-            lj_pair<ACCUM, ENERGY, VIRIAL>(
-                a, acc, sA, sB, t_i[ii], p_i[ii].w, g_i[ii],
-                make_float4(pj.x + sh.x - p_i[ii].x, pj.y + sh.y - p_i[ii].y,
-                            pj.z + sh.z - p_i[ii].z, pj.w),
-                jj, tj, f_i[ii][0], f_i[ii][1], f_i[ii][2], elj_i[ii], ec_i[ii], vir_i[ii]);
-          }
-        }
-      }
-      __syncwarp();
-    }
-#pragma unroll
-    for (int ii = 0; ii < kClusterSize; ++ii) {
-      if (ii >= ci.y) break;  // warp-uniform
-      const float fx = warp_sum(f_i[ii][0]), fy = warp_sum(f_i[ii][1]),
-                  fz = warp_sum(f_i[ii][2]);
-      float el = 0.f, ec = 0.f;
-      if (ENERGY) {
-        el = warp_sum(elj_i[ii]);
-        ec = warp_sum(ec_i[ii]);
-      }
-      if (VIRIAL) {
-#pragma unroll
-        for (int q = 0; q < 6; ++q) vir_i[ii][q] = warp_sum(vir_i[ii][q]);
-      }
-      if (lane == 0) {
-        add_force<ACCUM>(acc, ci.x + ii, fx, fy, fz);
-        if (ENERGY) add_energy<ACCUM>(acc, ci.x + ii, el + ec, el, ec);
-        if (VIRIAL) add_virial<ACCUM>(acc, ci.x + ii, vir_i[ii]);
-      }
-    }
-  }
-}
-
-template <int ACCUM, bool ENERGY, bool VIRIAL>
-static int launch_clusters3(const ClusterPairArgs& a, Accumulators& acc, cudaStream_t st) {
-  const size_t smem = sizeof(float) * a.n_types * (a.n_types + 1);
-  auto kern = k_lj_clusters<ACCUM, ENERGY, VIRIAL>;
-  static int sms = 0;
-  if (!sms) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, 0);
-  int per_sm = 1;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32 * kCWarps, smem);
-  per_sm = std::max(per_sm, 1);
-  if (a.blocks_per_sm > 0) per_sm = std::min(per_sm, a.blocks_per_sm);
-  kern<<<sms * per_sm, 32 * kCWarps, smem, st>>>(a, acc);
-  SNB_CUDA_TRY(cudaGetLastError());
-  return kOk;
-}
-
-template <int ACCUM>
-static int launch_clusters2(const ClusterPairArgs& a, Accumulators& acc, bool energy,
-                            bool virial, cudaStream_t st) {
-  if (energy && virial) return launch_clusters3<ACCUM, true, true>(a, acc, st);
-  if (energy) return launch_clusters3<ACCUM, true, false>(a, acc, st);
-  if (virial) return launch_clusters3<ACCUM, false, true>(a, acc, st);
-  return launch_clusters3<ACCUM, false, false>(a, acc, st);
-}
-
-int launch_pair_clusters(const ClusterPairArgs& a, Accumulators& acc, int accum,
-                         bool energy, bool virial, cudaStream_t st) {
-  return accum == kAccumFixed ? launch_clusters2<kAccumFixed>(a, acc, energy, virial, st)
-                              : launch_clusters2<kAccumFloat>(a, acc, energy, virial, st);
 }
 
 // ---------------------------------------------------------------------------
@@ -888,233 +560,6 @@ k_lj_soft(SoftArgs a, Accumulators acc, long long* dudl_total) {
     }
     if (VIRIAL) add_virial<ACCUM>(acc, i, vir);
   }
-}
-
-// Soft-core pair terms without dU/dlambda (the forms of k_lj_soft): force
-// over r, LJ and Coulomb energies.  alp_A = alpha lambda^p, alp_B = alpha
-// (1 - lambda)^p.
-__device__ __forceinline__ void soft_pair(const SoftArgs& a, float AA, float AB, float BA,
-                                          float BB, float r2, float qq, float alp_A,
-                                          float alp_B, float& fs, float& elj, float& ec) {
-  const float lam = a.lambda, lam_ = 1.0f - a.lambda;
-  const float r = sqrtf(r2);
-  if (BA * AA != 0.f || BA + AA == 0.f) {
-    const float ir2 = 1.0f / r2, ir6 = ir2 * ir2 * ir2;
-    fs = lam_ * (AB - AA * ir6) * ir6 * ir2 + lam * (BB - BA * ir6) * ir6 * ir2 -
-         coul_f(qq, a.beta, r);
-    elj = lam_ * lj_e(AA, AB, ir6) + lam * lj_e(BA, BB, ir6);
-    ec = coul_e(qq, a.beta, r);
-  } else {
-    const float sA = sc_sigma(AA, AB, a.sigma6, a.sigma6_min);
-    const float sB = sc_sigma(BA, BB, a.sigma6, a.sigma6_min);
-    const float r6 = r2 * r2 * r2;
-    const float rA = powf(r6 + alp_A * sA, 0.16666667f);
-    const float rB = powf(r6 + alp_B * sB, 0.16666667f);
-    const float r4 = r2 * r2;
-    const float iA2 = 1.0f / (rA * rA), iA6 = iA2 * iA2 * iA2;
-    const float iB2 = 1.0f / (rB * rB), iB6 = iB2 * iB2 * iB2;
-    const float flA = r4 * (AB - AA * iA6) * iA6 * iA6;
-    const float flB = r4 * (BB - BA * iB6) * iB6 * iB6;
-    const float bA = a.beta * rA, bB = a.beta * rB;
-    const float fcA =
-        qq * r4 * (expf(-bA * bA) * kTwoOverSqrtPi * a.beta + erfcf(bA) / rA) * iA6;
-    const float fcB =
-        qq * r4 * (expf(-bB * bB) * kTwoOverSqrtPi * a.beta + erfcf(bB) / rB) * iB6;
-    fs = lam_ * flA + lam * flB - (lam_ * fcA + lam * fcB);
-    ec = lam_ * coul_e(qq, a.beta, rA) + lam * coul_e(qq, a.beta, rB);
-    elj = lam_ * lj_e(AA, AB, iA6) + lam * lj_e(BA, BB, iB6);
-  }
-}
-
-// Soft-core LJ + direct Coulomb for the fused engine, in the two-phase row
-// scheme of k_lj_direct (scan to a shared hit list, then dense batches of
-// pair terms).  A pair whose end states carry the same LJ parameters
-// (A'_A == A'_B and B'_A == B'_B, as between unperturbed atoms) takes the
-// plain pair terms of lj_pair, to which the lambda mix of the two equal
-// forms reduces; the other pairs take soft_pair.  Energies and virial split
-// by global id as in k_lj_direct; no inter/intra split and no dU/dlambda
-// (the module's k_lj_soft provides those).
-template <int ACCUM, bool ENERGY, bool VIRIAL>
-__global__ void __launch_bounds__(256, 4)
-k_lj_soft_rows(SoftArgs a, Accumulators acc) {
-  constexpr int kScanU = 4;
-  extern __shared__ float sh_soft[];
-  __shared__ int hits_all[kWarps][kHitCap];
-  const int pA_n = a.n_types_A * (a.n_types_A + 1) / 2;
-  const int pB_n = a.n_types_B * (a.n_types_B + 1) / 2;
-  float* sAA = sh_soft;
-  float* sAB = sAA + pA_n;
-  float* sBA = sAB + pA_n;
-  float* sBB = sBA + pB_n;
-  for (int k = threadIdx.x; k < pA_n; k += blockDim.x) {
-    sAA[k] = a.AA[k];
-    sAB[k] = a.AB[k];
-  }
-  for (int k = threadIdx.x; k < pB_n; k += blockDim.x) {
-    sBA[k] = a.BA[k];
-    sBB[k] = a.BB[k];
-  }
-  __syncthreads();
-  const int lane = threadIdx.x & 31;
-  const int w = threadIdx.x >> 5;
-  int* hits = hits_all[w];
-  if (a.nl_flags && a.nl_flags[1]) return;  // list overflowed: rows not written
-  // pruned rows, as in k_lj_direct
-  const bool prune_pass = a.prune != nullptr && a.prune[0] != 0;
-  const bool use_inner = a.prune != nullptr && !prune_pass;
-  const int* __restrict__ cols = use_inner ? a.cols_in : a.cols;
-  const int* __restrict__ rcount = use_inner ? a.row_in_count : a.row_count;
-  const float alp_A = a.alpha * powf(a.lambda, a.p);
-  const float alp_B = a.alpha * powf(1.0f - a.lambda, a.p);
-  const int per_block = (a.n + gridDim.x - 1) / gridDim.x;
-  const int i_begin = blockIdx.x * per_block;
-  const int i_end = min(a.n, i_begin + per_block);
-  const unsigned lt = (1u << lane) - 1u;
-  // the plain-path constants of lj_pair
-  PairArgs pa;
-  pa.beta = a.beta;
-  pa.global = a.global;
-  for (int i = i_begin + w; i < i_end; i += kWarps) {
-    const float4 pi = a.pos[i];
-    const float3 ri = make_float3(pi.x, pi.y, pi.z);
-    const int2 pri = a.par[i];
-    const int tAi = pri.x & 0xffff, tBi = pri.x >> 16;
-    const int gi = ENERGY || VIRIAL ? a.global[i] : 0;
-    float fx = 0.f, fy = 0.f, fz = 0.f;
-    float e_lj = 0.f, e_c = 0.f;
-    float vir[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    const int k0 = a.row_start[i], k1 = k0 + rcount[i];
-    int kept = 0;  // prune pass: entries kept so far
-    for (int base = k0; base < k1;) {
-      int count = 0;
-      for (; base < k1 && count <= kHitCap - 32 * kScanU; base += 32 * kScanU) {
-        int jj[kScanU];
-#pragma unroll
-        for (int u = 0; u < kScanU; ++u) {
-          const int k = base + 32 * u + lane;
-          jj[u] = k < k1 ? cols[k] : -1;
-        }
-        float4 pp[kScanU];
-#pragma unroll
-        for (int u = 0; u < kScanU; ++u)
-          if (jj[u] >= 0) pp[u] = a.pos[jj[u]];
-#pragma unroll
-        for (int u = 0; u < kScanU; ++u) {
-          bool in = false, keep = false;
-          if (jj[u] >= 0) {
-            const float3 dr = min_image_fast<true>(make_float3(pp[u].x, pp[u].y, pp[u].z),
-                                                   ri, a.cell, a.rcell);
-            const float d2 = dr.x * dr.x + dr.y * dr.y + dr.z * dr.z;
-            in = d2 < a.cutoff2;
-            keep = d2 < a.prune2;
-          }
-          if (prune_pass) {  // warp-uniform
-            const unsigned mk = __ballot_sync(0xffffffffu, keep);
-            if (keep) a.cols_in[k0 + kept + __popc(mk & lt)] = jj[u];
-            kept += __popc(mk);
-          }
-          const unsigned m = __ballot_sync(0xffffffffu, in);
-          if (in) hits[count + __popc(m & lt)] = jj[u];
-          count += __popc(m);
-        }
-      }
-      __syncwarp();
-      for (int h = lane; h < count; h += 32) {
-        const int j = hits[h];
-        const float4 pj = a.pos[j];
-        const int2 prj = a.par[j];
-        const float3 dr = min_image_fast<true>(make_float3(pj.x, pj.y, pj.z), ri, a.cell,
-                                               a.rcell);
-        const int pA = lj_pair_index(tAi, prj.x & 0xffff);
-        const int pB = lj_pair_index(tBi, prj.x >> 16);
-        const float AA = sAA[pA], AB = sAB[pA], BA = sBA[pB], BB = sBB[pB];
-        if (AA == BA && AB == BB) {
-          // one table entry carries the pair's (equal) end-state parameters
-          lj_pair<ACCUM, ENERGY, VIRIAL>(pa, acc, sAA, sAB, tAi, pi.w, gi,
-                                         make_float4(dr.x, dr.y, dr.z, pj.w), j,
-                                         prj.x & 0xffff, fx, fy, fz, e_lj, e_c, vir);
-          continue;
-        }
-        const float r2 = dr.x * dr.x + dr.y * dr.y + dr.z * dr.z;
-        float fs, elj, ec;
-        soft_pair(a, AA, AB, BA, BB, r2, pi.w * pj.w, alp_A, alp_B, fs, elj, ec);
-        const float gx = fs * dr.x, gy = fs * dr.y, gz = fs * dr.z;
-        fx += gx;
-        fy += gy;
-        fz += gz;
-        add_force<ACCUM>(acc, j, -gx, -gy, -gz);
-        if (ENERGY || VIRIAL) {
-          const bool own_i = gi < a.global[j];
-          if (ENERGY) {
-            if (own_i) {
-              e_lj += elj;
-              e_c += ec;
-            } else {
-              add_energy<ACCUM>(acc, j, elj + ec, elj, ec);
-            }
-          }
-          if (VIRIAL) {
-            float v[6];
-            v[0] = -(gx * dr.x);
-            v[1] = -(gx * dr.y + gy * dr.x);
-            v[2] = -(gy * dr.y);
-            v[3] = -(gx * dr.z + gz * dr.x);
-            v[4] = -(gy * dr.z + gz * dr.y);
-            v[5] = -(gz * dr.z);
-            if (own_i) {
-#pragma unroll
-              for (int c = 0; c < 6; ++c) vir[c] += v[c];
-            } else {
-              add_virial<ACCUM>(acc, j, v);
-            }
-          }
-        }
-      }
-      __syncwarp();
-    }
-    if (prune_pass && lane == 0) {
-      a.row_in_count[i] = kept;
-      a.prune_ref[i] = pi;
-    }
-    fx = warp_sum(fx);
-    fy = warp_sum(fy);
-    fz = warp_sum(fz);
-    if (ENERGY) {
-      e_lj = warp_sum(e_lj);
-      e_c = warp_sum(e_c);
-    }
-    if (VIRIAL) {
-#pragma unroll
-      for (int c = 0; c < 6; ++c) vir[c] = warp_sum(vir[c]);
-    }
-    if (lane == 0) {
-      add_force<ACCUM>(acc, i, fx, fy, fz);
-      if (ENERGY) add_energy<ACCUM>(acc, i, e_lj + e_c, e_lj, e_c);
-      if (VIRIAL) add_virial<ACCUM>(acc, i, vir);
-    }
-  }
-}
-
-int launch_soft_rows(const SoftArgs& a, Accumulators& acc, bool energy, bool virial,
-                     cudaStream_t st) {
-  if (a.n <= 0) return kOk;
-  const size_t smem = sizeof(float) * (a.n_types_A * (a.n_types_A + 1) +
-                                       a.n_types_B * (a.n_types_B + 1));
-  using Kern = void (*)(SoftArgs, Accumulators);
-  Kern kern = energy && virial ? k_lj_soft_rows<kAccumFixed, true, true>
-              : energy         ? k_lj_soft_rows<kAccumFixed, true, false>
-              : virial         ? k_lj_soft_rows<kAccumFixed, false, true>
-                               : k_lj_soft_rows<kAccumFixed, false, false>;
-  if (smem > 48 * 1024) return fail(kNotSupported, "soft-core rows: type tables too large");
-  static int sms = 0;
-  if (!sms) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, 0);
-  int per_sm = 1;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32 * kWarps, smem);
-  per_sm = std::max(per_sm, 1);
-  const int blocks = std::max(1, std::min(sms * per_sm, ceil_div(a.n, kWarps)));
-  kern<<<blocks, 32 * kWarps, smem, st>>>(a, acc);
-  SNB_CUDA_TRY(cudaGetLastError());
-  return kOk;
 }
 
 template <int ACCUM>

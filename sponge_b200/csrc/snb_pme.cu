@@ -173,7 +173,7 @@ __global__ void k_pack_pme_bin(int n, const float3* __restrict__ crd,
                                TileGeom g, int* __restrict__ atom_tile,
                                int* __restrict__ atom_slot, int* __restrict__ tile_count,
                                float4* __restrict__ frq, int* __restrict__ upk,
-                               BatchView bv, const float3* __restrict__ img_off) {
+                               BatchView bv) {
   int s = blockIdx.x * blockDim.x + threadIdx.x;
   const bool active = s < n;
   int t = 0;
@@ -183,12 +183,7 @@ __global__ void k_pack_pme_bin(int n, const float3* __restrict__ crd,
     int i = perm ? perm[s] : s;
     float3 r = crd[i];
     float q = charge[i];
-    if (img_off) {
-      const float3 o = img_off[s];
-      pos[s] = make_float4(r.x - o.x, r.y - o.y, r.z - o.z, q);
-    } else {
-      pos[s] = make_float4(r.x, r.y, r.z, q);
-    }
+    pos[s] = make_float4(r.x, r.y, r.z, q);
     if (type_sorted) type_sorted[s] = type[i];
     int tile_begin = 0;
     if (BATCH) {
@@ -1184,9 +1179,9 @@ __global__ void k_pme_gather(int n, const float4* __restrict__ frq,
   if (active && ox == 0) {
     const int N = acc.n;
     if (ACCUM == kAccumFixed) {
-      red_add(acc.d_f + i, to_fixed_force(ax));
-      red_add(acc.d_f + N + i, to_fixed_force(ay));
-      red_add(acc.d_f + 2 * N + i, to_fixed_force(az));
+      red_add(acc.d_f + i * acc.fs, to_fixed_force(ax));
+      red_add(acc.d_f + i * acc.fs + acc.fc, to_fixed_force(ay));
+      red_add(acc.d_f + i * acc.fs + 2 * acc.fc, to_fixed_force(az));
     } else {
       atomicAdd(acc.d_ff + i, ax);
       atomicAdd(acc.d_ff + N + i, ay);
@@ -1665,18 +1660,17 @@ void pme_free(PME& p) {
 // Binning from caller-frame coordinates through a permutation, fused with
 // the pack of the pair kernel's input (pos, type_sorted may be null).
 int pme_pack_bin(PME& p, int n, const float3* crd, const float* charge, const int* type,
-                 const int* perm, float4* pos, int* type_sorted, cudaStream_t st,
-                 const float3* img_off) {
+                 const int* perm, float4* pos, int* type_sorted, cudaStream_t st) {
   if (n != p.n) return fail(kBadInput, "PME: atom count differs from Initial");
   TileGeom g{p.K[0], p.K[1], p.K[2], p.T, p.nt[0], p.nt[1], p.nt[2], p.rcell};
   if (p.bv.nsys > 0)
     k_pack_pme_bin<true><<<ceil_div(n, 256), 256, 0, st>>>(
         n, crd, charge, type, perm, pos, type_sorted, g, p.d_atom_tile, p.d_atom_slot,
-        p.d_tile_count, p.d_frq, p.d_upk, p.bv, img_off);
+        p.d_tile_count, p.d_frq, p.d_upk, p.bv);
   else
     k_pack_pme_bin<false><<<ceil_div(n, 256), 256, 0, st>>>(
         n, crd, charge, type, perm, pos, type_sorted, g, p.d_atom_tile, p.d_atom_slot,
-        p.spread_atomic ? nullptr : p.d_tile_count, p.d_frq, p.d_upk, p.bv, img_off);
+        p.spread_atomic ? nullptr : p.d_tile_count, p.d_frq, p.d_upk, p.bv);
   SNB_CUDA_TRY(cudaGetLastError());
   return kOk;
 }
@@ -1925,9 +1919,9 @@ __global__ void k_excluded(int n, const float3* __restrict__ crd,
     fz += gz;
     int sj = map ? map[j] : j;
     if (ACCUM == kAccumFixed) {
-      red_add(acc.d_f + sj, -to_fixed_force(gx));
-      red_add(acc.d_f + N + sj, -to_fixed_force(gy));
-      red_add(acc.d_f + 2 * N + sj, -to_fixed_force(gz));
+      red_add(acc.d_f + sj * acc.fs, -to_fixed_force(gx));
+      red_add(acc.d_f + sj * acc.fs + acc.fc, -to_fixed_force(gy));
+      red_add(acc.d_f + sj * acc.fs + 2 * acc.fc, -to_fixed_force(gz));
     } else {
       atomicAdd(acc.d_ff + sj, -gx);
       atomicAdd(acc.d_ff + N + sj, -gy);
@@ -1945,9 +1939,9 @@ __global__ void k_excluded(int n, const float3* __restrict__ crd,
   }
   int si = map ? map[i] : i;
   if (ACCUM == kAccumFixed) {
-    red_add(acc.d_f + si, to_fixed_force(fx));
-    red_add(acc.d_f + N + si, to_fixed_force(fy));
-    red_add(acc.d_f + 2 * N + si, to_fixed_force(fz));
+    red_add(acc.d_f + si * acc.fs, to_fixed_force(fx));
+    red_add(acc.d_f + si * acc.fs + acc.fc, to_fixed_force(fy));
+    red_add(acc.d_f + si * acc.fs + 2 * acc.fc, to_fixed_force(fz));
     if (ENERGY) red_add(acc.d_e + si, to_fixed_energy(e));
     if (VIRIAL)
       for (int c = 0; c < 6; ++c) red_add(acc.d_v + c * N + si, to_fixed_energy(v[c]));

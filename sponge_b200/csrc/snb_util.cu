@@ -145,10 +145,13 @@ int scan_exclusive(const int* in, int* out, int n, int* total_out,
 }
 
 // ---------------------------------------------------------------------------
-int acc_init(Accumulators& a, int n) {
+int acc_init(Accumulators& a, int n, bool by_atom) {
   a.n = n;
   size_t N = n > 0 ? n : 1;
-  SNB_CUDA_TRY(cudaMalloc(&a.d_f, sizeof(long long) * 3 * N));
+  a.fs = by_atom ? 4 : 1;
+  a.fc = by_atom ? 1 : n;
+  a.f_len = (by_atom ? 4 : 3) * N;
+  SNB_CUDA_TRY(cudaMalloc(&a.d_f, sizeof(long long) * a.f_len));
   SNB_CUDA_TRY(cudaMalloc(&a.d_e, sizeof(long long) * 3 * N));
   a.d_elj = a.d_e + N;
   a.d_ec = a.d_e + 2 * N;
@@ -160,7 +163,7 @@ int acc_init(Accumulators& a, int n) {
   SNB_CUDA_TRY(cudaMalloc(&a.d_feaux, sizeof(float) * 2 * N));
   SNB_CUDA_TRY(cudaMemset(a.d_eaux, 0, sizeof(long long) * 2 * N));
   SNB_CUDA_TRY(cudaMemset(a.d_feaux, 0, sizeof(float) * 2 * N));
-  SNB_CUDA_TRY(cudaMemset(a.d_f, 0, sizeof(long long) * 3 * N));
+  SNB_CUDA_TRY(cudaMemset(a.d_f, 0, sizeof(long long) * a.f_len));
   SNB_CUDA_TRY(cudaMemset(a.d_e, 0, sizeof(long long) * 3 * N));
   SNB_CUDA_TRY(cudaMemset(a.d_v, 0, sizeof(long long) * 6 * N));
   SNB_CUDA_TRY(cudaMemset(a.d_ff, 0, sizeof(float) * 3 * N));
@@ -185,7 +188,7 @@ int launch_zero_acc(Accumulators& a, int accum, bool energy, bool virial,
                     cudaStream_t st) {
   size_t N = a.n > 0 ? a.n : 1;
   if (accum == kAccumFixed) {
-    SNB_CUDA_TRY(cudaMemsetAsync(a.d_f, 0, sizeof(long long) * 3 * N, st));
+    SNB_CUDA_TRY(cudaMemsetAsync(a.d_f, 0, sizeof(long long) * a.f_len, st));
     if (energy) SNB_CUDA_TRY(cudaMemsetAsync(a.d_e, 0, sizeof(long long) * 3 * N, st));
     if (virial) SNB_CUDA_TRY(cudaMemsetAsync(a.d_v, 0, sizeof(long long) * 6 * N, st));
   } else {
@@ -201,26 +204,20 @@ int launch_zero_acc(Accumulators& a, int accum, bool energy, bool virial,
 __global__ void k_pack(int n, const float3* __restrict__ crd,
                        const float* __restrict__ charge,
                        const int* __restrict__ type, const int* __restrict__ perm,
-                       float4* __restrict__ pos, int* __restrict__ type_sorted,
-                       const float3* __restrict__ img_off) {
+                       float4* __restrict__ pos, int* __restrict__ type_sorted) {
   int s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= n) return;
   int i = perm ? perm[s] : s;
-  float3 r = crd[i];
-  if (img_off) {
-    const float3 o = img_off[s];
-    r = make_float3(r.x - o.x, r.y - o.y, r.z - o.z);
-  }
+  const float3 r = crd[i];
   pos[s] = make_float4(r.x, r.y, r.z, charge[i]);
   if (type_sorted) type_sorted[s] = type[i];
 }
 
 int launch_pack(int n, const float3* crd, const float* charge, const int* type,
-                const int* perm, float4* pos, int* type_sorted, cudaStream_t st,
-                const float3* img_off) {
+                const int* perm, float4* pos, int* type_sorted, cudaStream_t st) {
   if (n <= 0) return kOk;
   k_pack<<<ceil_div(n, 256), 256, 0, st>>>(n, crd, charge, type, perm, pos,
-                                          type_sorted, img_off);
+                                          type_sorted);
   SNB_CUDA_TRY(cudaGetLastError());
   return kOk;
 }
@@ -237,12 +234,13 @@ __global__ void k_unpack(int n, const int* __restrict__ map, Accumulators a,
   const int N = a.n;
   float fx, fy, fz;
   if (ACCUM == kAccumFixed) {
-    fx = (float)((double)a.d_f[s] * kForceScaleInv);
-    fy = (float)((double)a.d_f[N + s] * kForceScaleInv);
-    fz = (float)((double)a.d_f[2 * N + s] * kForceScaleInv);
-    a.d_f[s] = 0;
-    a.d_f[N + s] = 0;
-    a.d_f[2 * N + s] = 0;
+    long long* f = a.d_f + s * a.fs;
+    fx = (float)((double)f[0] * kForceScaleInv);
+    fy = (float)((double)f[a.fc] * kForceScaleInv);
+    fz = (float)((double)f[2 * a.fc] * kForceScaleInv);
+    f[0] = 0;
+    f[a.fc] = 0;
+    f[2 * a.fc] = 0;
   } else {
     fx = a.d_ff[s];
     fy = a.d_ff[N + s];

@@ -171,23 +171,23 @@ __global__ void k_vatom_spread_fixed(int begin, int end, const VRecord* __restri
   const VRecord r = rec[t];
   const int N = acc.n;
   const int sv = map ? map[r.v] : r.v;
-  const float3 F = make_float3((float)((double)acc.d_f[sv] * kForceScaleInv),
-                               (float)((double)acc.d_f[N + sv] * kForceScaleInv),
-                               (float)((double)acc.d_f[2 * N + sv] * kForceScaleInv));
+  const float3 F = make_float3((float)((double)acc.d_f[sv * acc.fs] * kForceScaleInv),
+                               (float)((double)acc.d_f[sv * acc.fs + acc.fc] * kForceScaleInv),
+                               (float)((double)acc.d_f[sv * acc.fs + 2 * acc.fc] * kForceScaleInv));
   float3 fa, fb, fc;
   if (!v_split(r, F, crd, cell, rcell, &fa, &fb, &fc)) atomicCAS(err, 0, 1 + t);
   auto add = [&](int atom, float3 v) {
     const int s = map ? map[atom] : atom;
-    red_add(acc.d_f + s, to_fixed_force(v.x));
-    red_add(acc.d_f + N + s, to_fixed_force(v.y));
-    red_add(acc.d_f + 2 * N + s, to_fixed_force(v.z));
+    red_add(acc.d_f + s * acc.fs, to_fixed_force(v.x));
+    red_add(acc.d_f + s * acc.fs + acc.fc, to_fixed_force(v.y));
+    red_add(acc.d_f + s * acc.fs + 2 * acc.fc, to_fixed_force(v.z));
   };
   add(r.a, fa);
   if (r.type >= 1) add(r.b, fb);
   if (r.type >= 2) add(r.c, fc);
-  acc.d_f[sv] = 0;
-  acc.d_f[N + sv] = 0;
-  acc.d_f[2 * N + sv] = 0;
+  acc.d_f[sv * acc.fs] = 0;
+  acc.d_f[sv * acc.fs + acc.fc] = 0;
+  acc.d_f[sv * acc.fs + 2 * acc.fc] = 0;
 }
 
 }  // namespace snb

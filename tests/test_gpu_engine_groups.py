@@ -1,0 +1,122 @@
+"""The engine's grouped rows (k_group_search, k_lj_groups) where they can go
+wrong: boxes so small that each pair is imaged by itself, groups of every size
+from one atom to eight, rows of less than a batch and of several, a cutoff at
+which beta r leaves the erfc polynomial, more than two exclusions per atom, and
+charges and LJ types that differ inside a group.
+
+The pair set must be the oracle's bit for bit.  Forces: each pair's terms are
+32-bit (relative error below 1.1e-6, the erfc polynomial's), summed in 32 bits
+over at most 64 partners of a lane, so 1e-5 relative RMS against FP64 leaves a
+factor of five; energies within 2e-6, as in test_gpu_engine.py."""
+
+import ctypes
+import dataclasses
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def g():
+    import torch
+    assert torch.cuda.is_available(), "GPU tests need CUDA"
+    from tests import gpu_helpers
+    return gpu_helpers
+
+
+def _pairs(g, e):
+    import torch
+    lib = g.capi.load()
+    cnt = ctypes.c_longlong(0)
+    g.capi.check(lib.snb_engine_stats(e, None, ctypes.byref(cnt), g.stream()), "stats")
+    n = cnt.value
+    pi = torch.empty(max(n, 1), dtype=torch.int32, device="cuda")
+    pj = torch.empty(max(n, 1), dtype=torch.int32, device="cuda")
+    got = ctypes.c_longlong(0)
+    g.capi.check(lib.snb_engine_export_pairs(e, g.ptr(pi), g.ptr(pj), n, ctypes.byref(got),
+                                             g.stream()), "export")
+    assert got.value == n
+    p = np.stack([pi[:n].cpu().numpy(), pj[:n].cpu().numpy()], 1).astype(np.int64)
+    return p[np.lexsort((p[:, 1], p[:, 0]))]
+
+
+def _check(g, oracle, s, cutoff, tol=1e-5):
+    import torch
+    from sponge_b200 import systems
+    lib = g.capi.load()
+    e = g.engine_create(s, cutoff, PM_Direct_Tolerance=tol)
+    crd = g.dev(s.crd.reshape(-1), np.float32)
+    frc = torch.zeros(3 * s.n, dtype=torch.float32, device="cuda")
+    only = torch.zeros(3 * s.n, dtype=torch.float32, device="cuda")
+    tot = torch.zeros(16, dtype=torch.float64, device="cuda")
+    try:
+        g.capi.check(lib.snb_engine_force(e, g.ptr(crd), g.ptr(frc), 0, 1, 1, g.ptr(tot),
+                                          g.stream()), "engine_force")
+        g.capi.check(lib.snb_engine_force(e, g.ptr(crd), g.ptr(only), 1, 0, 0, None, g.stream()),
+                     "engine_force")
+        got = _pairs(g, e)
+    finally:
+        lib.snb_engine_destroy(e)
+    rs, cols = oracle.nl_pairs_system(s, cutoff, 2.0)
+    assert np.array_equal(got, g.csr_to_pairs(rs, cols))
+    beta = oracle.get_beta(cutoff, tol)
+    d, x = oracle.direct_f64(s, cutoff, beta, rs, cols), oracle.excluded_f64(s, beta)
+    p = oracle.pme_f64(s, (systems.fft_size(s.box),) * 3, beta)
+    want = d["frc"] + x["frc"] + p["frc"]
+    assert g.rel_rms(frc.cpu().numpy().reshape(s.n, 3), want) <= 1e-5
+    assert g.rel_rms(only.cpu().numpy().reshape(s.n, 3), want) <= 1e-5
+    t = tot.cpu().numpy()
+    assert abs(t[0] - d["lj_energy"].sum()) <= 2e-6 * np.abs(d["lj_energy"]).sum()
+    assert abs(t[2] - d["coulomb_energy"].sum()) <= 2e-6 * np.abs(d["coulomb_energy"]).sum()
+    vir = d["virial"].sum(0) + x["virial"].sum(0) + p["virial"]
+    lrc = oracle.lrc_factor(s, cutoff) / float(np.float32(s.box)) ** 3
+    vir[[0, 2, 5]] += 2 * lrc
+    assert np.abs(t[8:14] - vir).max() <= 2e-6 * np.abs(vir).max()
+
+
+@pytest.mark.parametrize("waters,cutoff,tol", [
+    (200, 8.0, 1e-5),    # half the box 9.07 A: every pair imaged, 3 cells per axis
+    (231, 9.0, 1e-5),    # the cutoff just below half the box
+    (700, 7.3, 1e-5),    # 5 cells per axis: trimmed runs, some groups imaged
+    (1500, 9.0, 1e-9),   # beta * cutoff = 4.3: beyond the polynomial
+    (2600, 6.1, 1e-5),   # narrow cells: groups of a few atoms
+])
+def test_groups_match_fp64(g, oracle, waters, cutoff, tol):
+    from sponge_b200 import systems
+    s = systems.water_box(waters, seed=waters, ion_pairs=None)
+    _check(g, oracle, s, cutoff, tol)
+
+
+def test_sparse_and_dense_cells(g, oracle):
+    """Most waters in one corner: empty cells, cells of one molecule and cells
+    of many groups; rows from empty to regrown."""
+    from sponge_b200 import systems
+    s = systems.water_box(900, seed=5)
+    rng = np.random.default_rng(5)
+    keep = np.ones(s.n, bool)
+    o = s.crd[::3] - np.floor(s.crd[::3] / s.box) * s.box
+    far = (o.max(1) > 0.55 * s.box) & (rng.random(len(o)) < 0.93)
+    keep = np.repeat(~far, 3)
+    _check(g, oracle, systems._subset(s, keep), 6.5)
+
+
+def test_many_exclusions_and_types(g, oracle):
+    """Chains of 24 waters excluded from one another (up to 71 partners, beyond
+    the 16 that the build keeps per atom) and four LJ types dealt out at
+    random."""
+    from sponge_b200 import systems
+    s = systems.water_box(1000, seed=8)
+    rng = np.random.default_rng(8)
+    lists = []
+    for i in range(s.n):
+        end = min(s.n, (i // 72 + 1) * 72)
+        lists.append(np.arange(i + 1, end) if (i // 72) % 3 == 0 else
+                     np.arange(i + 1, (i // 3 + 1) * 3))
+    numbers = np.array([len(x) for x in lists], np.int32)
+    start = np.concatenate([[0], np.cumsum(numbers)[:-1]]).astype(np.int32)
+    s = dataclasses.replace(s, excl_start=start, excl_numbers=numbers,
+                            excl_list=np.concatenate(lists).astype(np.int32))
+    s.lj_type[::3] = rng.choice([0, 2, 3], len(s.lj_type[::3]))
+    _check(g, oracle, s, 7.0)
