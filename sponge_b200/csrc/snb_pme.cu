@@ -498,11 +498,14 @@ k_pme_spread(TileGeom g, const int* __restrict__ tile_start,
   }
 }
 
-// The same grid by global atomics: 16 lanes per atom, lane (ox, oy) adds
-// the four points of its z line in int64 fixed point (the products formed
-// in the tile path's order, so every point gets the same integers; integer
-// sums do not depend on their order).  Atoms in the pair kernel's sorted
-// order, so a warp's two atoms are neighbours.
+// The same grid by global atomics: 16 lanes per atom, lane (oy, oz) adds one
+// point of each of the four x planes in int64 fixed point (the products
+// formed in the tile path's order, so every point gets the same integers;
+// integer sums do not depend on their order).  Four consecutive lanes take
+// the four points of a z line, which lie in one or two 32-byte sectors, so an
+// atom costs about 28 sector updates in L2, where a lane per line would cost
+// 64.  Atoms in the pair kernel's sorted order, so a warp's two atoms are
+// neighbours.
 __global__ void __launch_bounds__(256)
 k_pme_spread_red(int n, const float4* __restrict__ frq, const int* __restrict__ upk,
                  TileGeom g, long long* __restrict__ Q64) {
@@ -512,25 +515,27 @@ k_pme_spread_red(int n, const float4* __restrict__ frq, const int* __restrict__ 
   const float4 f = frq[i];
   const int up = upk[i];
   const int ux = up >> 20, uy = (up >> 10) & 1023, uz = up & 1023;
-  const int ox = l >> 2, oy = l & 3;
+  const int oy = l >> 2, oz = l & 3;
   float wx[4], wy[4], wz[4];
   bspline4(f.x, wx);
   bspline4(f.y, wy);
   bspline4(f.z, wz);
+  const float wyl = oy < 2 ? (oy == 0 ? wy[0] : wy[1]) : (oy == 2 ? wy[2] : wy[3]);
+  const float wzl = oz < 2 ? (oz == 0 ? wz[0] : wz[1]) : (oz == 2 ? wz[2] : wz[3]);
   const float qs = f.w * kGridScale;
-  const float wxy = qs * wx[ox] * wy[oy];
-  int px = ux - ox;
-  px += px < 0 ? g.K0 : 0;
   int py = uy - oy;
   py += py < 0 ? g.K1 : 0;
-  unsigned long long* row =
-      reinterpret_cast<unsigned long long*>(Q64) + ((size_t)px * g.K1 + py) * g.K2;
+  int pz = uz - oz;
+  pz += pz < 0 ? g.K2 : 0;
+  unsigned long long* at =
+      reinterpret_cast<unsigned long long*>(Q64) + (size_t)py * g.K2 + pz;
+  const size_t plane = (size_t)g.K1 * g.K2;
 #pragma unroll
-  for (int oz = 0; oz < 4; ++oz) {
-    int pz = uz - oz;
-    pz += pz < 0 ? g.K2 : 0;
-    const long long c = __float2int_rn(wxy * wz[oz]);
-    atomicAdd(row + pz, static_cast<unsigned long long>(c));
+  for (int ox = 0; ox < 4; ++ox) {
+    int px = ux - ox;
+    px += px < 0 ? g.K0 : 0;
+    const long long c = __float2int_rn(qs * wx[ox] * wyl * wzl);
+    atomicAdd(at + px * plane, static_cast<unsigned long long>(c));
   }
 }
 
