@@ -1080,7 +1080,7 @@ static int engine_finish_create(snb_engine* e, int n, int n_types, const int* h_
                                 const float* h_A, const float* h_B, const float* h_charge,
                                 const int* h_es, const int* h_en, const int* h_el,
                                 int n_excl) {
-  int rc = acc_init(e->acc, n, e->nl.groups);
+  int rc = acc_init(e->acc, n, e->accum == kAccumFixed);
   if (rc) return rc;
   LJParams& p = e->lj;
   p.n_types = n_types;
