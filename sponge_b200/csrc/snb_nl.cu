@@ -544,8 +544,10 @@ __device__ __forceinline__ float span_gap(int o, float lo, float hi) {
 // evaluations of a row remain, against 115 in the order of the cells (the
 // pair kernel: 161 us, against 167 us with 16 even bins and 173 us with 10).
 //
-// One rebuild of the 99,639-atom box takes 0.30 ms where the search of a row
-// per atom took 0.49 ms.
+// One rebuild of the 99,639-atom box takes 0.45 ms where the search of a row
+// per atom took 0.49 ms; of a 648-atom box, whose 90 groups leave the chip
+// idle, it takes about 25 us more than that.  Loading the candidates a batch
+// ahead made no difference, one warp per block (fewer in flight) doubled it.
 constexpr int kGroupBuf = 1024;
 constexpr int kGroupSearchWarps = 4;
 
