@@ -1118,22 +1118,17 @@ def run_ours(args):
             plain["speedup_vs_plain"] = plain["this_engine_ns_per_day"] / plain["ns_per_day"]
 
     # roofline of the dominant kernel (the pair kernel), HBM view.  Per
-    # launch, averaged over the profiled steps: the list entries scanned
-    # (the full rows on a prune pass, the kept entries otherwise), the
-    # positions, forces and row counts, and on a prune pass the kept entries
-    # written with the rows' counts and positions
+    # launch: the grouped rows' entries that the last prune pass kept (4 bytes
+    # each; a pass takes about a quarter more), the positions, types and forces
     pair_ms = float(phases[2])
     listed = int(pairs.value)
     prof_prunes = int(pq1.value - pq0.value)
-    f_prune = prof_prunes / max(1, args.profile_steps) if kept.value > 0 else 1.0
-    kept_n = int(kept.value) if kept.value > 0 else listed
-    scanned = f_prune * listed + (1.0 - f_prune) * kept_n
-    alg_bytes = (4 * scanned + 16 * n + 24 * n + 4 * (n + 1) + 4 * n
-                 + (f_prune * (4 * kept_n + 20 * n) if kept.value > 0 else 0.0))
+    scanned = int(kept.value) if kept.value > 0 else listed // 5
+    alg_bytes = 4 * scanned + 20 * n + 24 * n
     peak, peak_kind = measured_peaks()
     achieved = alg_bytes / (pair_ms * 1e-3) / 1e9
     traffic = committed_traffic()
-    roofline = {"bound": "hbm", "kernel": "k_lj_direct", "achieved": achieved,
+    roofline = {"bound": "hbm", "kernel": "k_lj_groups", "achieved": achieved,
                 "peak": peak, "peak_kind": peak_kind, "unit": "GB/s",
                 "frac": achieved / peak,
                 "traffic": (traffic["dram_bytes_per_launch"] if traffic else None),
@@ -1141,9 +1136,10 @@ def run_ours(args):
                 "entries_scanned_per_launch": scanned, "prune_passes_profiled": prof_prunes,
                 "profiled_steps": args.profile_steps}
     # FP32-pipe view: 47 flops per in-cutoff pair (force only) + 10 per other
-    # scanned entry; in-cutoff count from the oracle-free density estimate
+    # pair of an entry and the about seven atoms of its group; in-cutoff count
+    # from the density
     in_cut = listed * (CUTOFF / (CUTOFF + SKIN)) ** 3
-    flops = 47 * in_cut + 10 * (scanned - in_cut)
+    flops = 47 * in_cut + 10 * max(0.0, 7.0 * scanned - in_cut)
     roofline["fp32_tflops"] = flops / (pair_ms * 1e-3) / 1e12
 
     cpu_base = None
