@@ -363,7 +363,7 @@ k_lj_groups(GroupArgs a, Accumulators acc) {
 
     for (int c0 = b0; c0 < b1; c0 += 32) {
       // the next (up to) 32 batches: lane k holds the i atoms of batch c0 + k
-      const unsigned mine = c0 + lane < b1 ? (kept ? (unsigned)bytes[c0 + lane] : own_bits) : 0u;
+      const unsigned mine = c0 + lane < b1 ? (kept ? (unsigned)bytes[c0 + lane] : 0xffu) : 0u;
       unsigned todo = __ballot_sync(0xffffffffu, mine != 0u);
       if (todo == 0u) continue;
       // entries are loaded two batches ahead, partners one ahead

@@ -166,12 +166,11 @@ struct NeighborList {
   // atoms of one cell, whose atoms follow a path up and down the cell's four
   // xy quarter columns.  Row g lists the partner atoms with a pair within r_l
   // of group g as (sorted index << 8 | mask of the group's atoms), nearest
-  // first.  A cell's groups are numbered from cell_start / gsize + cell,
+  // first.  A cell's groups are numbered from cell_start / kGroupSize + cell,
   // which leaves room for each cell's last, shorter group, so the numbers of
   // a batch's systems do not depend on one another.  With groups the per-atom
   // rows above are not allocated.
   bool groups = false;
-  int gsize = 8;                 // atoms a group may hold (at most kGroupSize)
   int max_groups = 0;
   int* d_atom_key = nullptr;     // [n] caller frame: order key inside the cell
   int2* d_group = nullptr;       // [max_groups] {first sorted atom, atom count}

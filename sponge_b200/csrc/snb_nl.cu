@@ -173,7 +173,7 @@ __global__ void k_bin_scatter(int n, const int* __restrict__ atom_cell,
 __global__ void k_cell_order(int ncell, const int* __restrict__ cell_start,
                              const int* __restrict__ unsorted,
                              int* __restrict__ perm, const int* flags,
-                             const int* __restrict__ key, int2* __restrict__ group, int gsize,
+                             const int* __restrict__ key, int2* __restrict__ group,
                              const unsigned char* __restrict__ box_need,
                              const int* __restrict__ cell_sys) {
   if (flags[kFlagNeed] == 0) return;
@@ -183,9 +183,9 @@ __global__ void k_cell_order(int ncell, const int* __restrict__ cell_start,
   if (!box_rebuilds(box_need, cell_sys, c)) return;
   int a = cell_start[c], b = cell_start[c + 1];
   if (group) {
-    const int ng = (b - a + gsize - 1) / gsize;
+    const int ng = (b - a + kGroupSize - 1) / kGroupSize;
     const int per = ng > 0 ? (b - a + ng - 1) / ng : 0;
-    const int id0 = a / gsize + c, id1 = b / gsize + c + 1;
+    const int id0 = a / kGroupSize + c, id1 = b / kGroupSize + c + 1;
     for (int t = lane; t < id1 - id0; t += 32)
       group[id0 + t] = make_int2(min(a + t * per, b - 1), max(0, min(per, b - a - t * per)));
   }
@@ -545,8 +545,8 @@ __device__ __forceinline__ float span_gap(int o, float lo, float hi) {
 // pair kernel: 161 us, against 167 us with 16 even bins and 173 us with 10).
 //
 // One rebuild of the 99,639-atom box takes 0.45 ms where the search of a row
-// per atom took 0.49 ms; a small box's few groups leave the chip idle (648
-// atoms: 28 us against 17 us, 9,000: about 55 us against 27 us).  Loading the candidates a batch
+// per atom took 0.49 ms; of a 648-atom box, whose 90 groups leave the chip
+// idle, it takes about 25 us more than that.  Loading the candidates a batch
 // ahead made no difference, one warp per block (fewer in flight) doubled it.
 constexpr int kGroupBuf = 1024;
 constexpr int kGroupSearchWarps = 4;
@@ -1178,13 +1178,6 @@ int nl_init_batch(NeighborList& nl, int n, float cutoff, float skin,
   return nl_alloc(nl, n, 0, runs, geom, counts, max_per, all_balanced, groups);
 }
 
-// Up to this many atoms a group holds half as many: the number of groups is
-// what the search of a small box is short of (one warp each).  A rebuild of
-// the 648-atom box takes 28 us against 38 us with groups of eight, the MD step
-// of a 3,000-atom box is the same with either; on 9,000 atoms the step is
-// 1.6 us longer with the smaller groups.
-constexpr int kSmallBox = 4000;
-
 static void groups_free(NeighborList& nl) {
   cudaFree(nl.d_atom_key);
   cudaFree(nl.d_group);
@@ -1203,7 +1196,7 @@ static int groups_alloc(NeighborList& nl) {
   const bool pruned = nl.d_gmask != nullptr;
   groups_free(nl);
   nl.gcap = (std::max(nl.gcap, 32) + 31) & ~31;
-  nl.max_groups = nl.n / nl.gsize + nl.ncell;
+  nl.max_groups = nl.n / kGroupSize + nl.ncell;
   const size_t G = nl.max_groups;
   SNB_CUDA_TRY(cudaMalloc(&nl.d_atom_key, sizeof(int) * nl.n));
   SNB_CUDA_TRY(cudaMalloc(&nl.d_group, sizeof(int2) * G));
@@ -1260,7 +1253,6 @@ static int nl_alloc(NeighborList& nl, int n, long long initial_capacity,
   }
   if (groups && n < kGroupMaxAtoms) {
     nl.groups = true;
-    nl.gsize = n <= kSmallBox ? kGroupSize / 2 : kGroupSize;
     // the row of a group of reach about 2 A: the half sphere of r_l + 2 A
     const double rl = sqrt((double)nl.rl2), s = (rl + 2.0) / rl;
     const double mean = max_per_atom * s * s * s;
@@ -1394,7 +1386,7 @@ int nl_regrid(NeighborList& nl, const float* cell6) {
   nl.wy = c.a22 / nl.Ny;
   nl.iwz = nl.Nz / c.a33;
   nl.generation = 0;  // the next update rebuilds
-  if (nl.groups && nl.max_groups != nl.n / nl.gsize + nl.ncell) {
+  if (nl.groups && nl.max_groups != nl.n / kGroupSize + nl.ncell) {
     SNB_CUDA_TRY(cudaDeviceSynchronize());
     return groups_alloc(nl);
   }
@@ -1499,8 +1491,7 @@ int nl_rebuild(NeighborList& nl, const float* crd_f, const int* atom_local,
       excl_list, excl_numbers, excl_count, nl.d_excl_partner, nl.d_flags, need, sys_of);
   k_cell_order<<<ceil_div(nl.ncell, 8), 256, 0, st>>>(nl.ncell, nl.d_cell_start,
                                                       nl.d_unsorted, nl.d_perm,
-                                                      nl.d_flags, key, nl.d_group, nl.gsize,
-                                                      need,
+                                                      nl.d_flags, key, nl.d_group, need,
                                                       cell_sys);
   k_fill_sorted<<<ceil_div(n, 256), 256, 0, st>>>(n, nl.d_perm, crd, atom_local,
                                                   nl.d_inv_perm, nl.d_global,
