@@ -101,6 +101,20 @@ struct snb_settle {
   Settle s;
 };
 
+// A soft-core module's tables and packed types as the grouped pair kernel reads
+// them (row strides n_types of the module they were made from).
+struct SoftTables {
+  float2* a = nullptr;
+  float2* b = nullptr;
+  int* type = nullptr;
+  void release() {
+    cudaFree(a);
+    cudaFree(b);
+    cudaFree(type);
+    *this = SoftTables();
+  }
+};
+
 struct snb_engine {
   snb_options opt;
   int n = 0;
@@ -160,9 +174,7 @@ struct snb_engine {
   // types (caller frame) of the plain LJ and of the soft-core module in use
   float2* d_lj_tab = nullptr;
   int* d_gtype = nullptr;
-  float2* d_soft_a = nullptr;
-  float2* d_soft_b = nullptr;
-  int* d_soft_type = nullptr;
+  SoftTables soft_tab;  // of `soft`; empty where its type tables are too large
   bool cluster_form = false;    // what snb_engine_list_form reports
   // launch shapes: blocks per SM is tuned; the others are settings of pair
   // kernels that are gone, kept for callers that set and read them back
@@ -1018,15 +1030,17 @@ static std::vector<char> types_without_lj(int T, const float* A, const float* B)
   return none;
 }
 
-// The soft-core module's tables and packed types for the grouped pair kernel.
 // An atom is marked (sign bit) unless every pair of unmarked atoms has equal
 // end states, so that a pair of two unmarked atoms takes the plain terms: its
 // (A type, B type) joins the unmarked ones, in order of how many atoms carry
 // it, when its pairs with all of them (and itself) are equal in both states.
-static int engine_soft_tables(snb_engine* e, const snb_lj_soft* h) {
-  const int nA = h->nA, nB = h->nB, n = e->n;
+// Type tables above 48 KB give no tables and their steps are refused, as ever:
+// the packed types have 15 bits each, and the marking compares every kind of
+// atom with every other.
+static int engine_soft_tables(const snb_lj_soft* h, SoftTables* out) {
+  const int nA = h->nA, nB = h->nB, n = h->n;
   const size_t smem = sizeof(float) * ((size_t)nA * (nA + 1) + (size_t)nB * (nB + 1));
-  if (smem > 48 * 1024) return kOk;  // refused when a step runs
+  if (smem > 48 * 1024) return kOk;
   const int pA = nA * (nA + 1) / 2, pB = nB * (nB + 1) / 2;
   std::vector<float> AA(pA), AB(pA), BA(pB), BB(pB);
   std::vector<int2> par(n);
@@ -1067,12 +1081,18 @@ static int engine_soft_tables(snb_engine* e, const snb_lj_soft* h) {
     if (marked[tA * nB + tB]) v |= 0x80000000u;
     packed[i] = (int)v;
   }
-  int rc = upload_pair_table(nA, AA.data(), AB.data(), &e->d_soft_a);
-  if (!rc) rc = upload_pair_table(nB, BA.data(), BB.data(), &e->d_soft_b);
-  if (rc) return rc;
-  if (!e->d_soft_type) SNB_CUDA_TRY(cudaMalloc(&e->d_soft_type, sizeof(int) * n));
-  SNB_CUDA_TRY(cudaMemcpy(e->d_soft_type, packed.data(), sizeof(int) * n,
-                          cudaMemcpyHostToDevice));
+  SoftTables t;
+  int rc = upload_pair_table(nA, AA.data(), AB.data(), &t.a);
+  if (!rc) rc = upload_pair_table(nB, BA.data(), BB.data(), &t.b);
+  if (!rc && (cudaMalloc(&t.type, sizeof(int) * n) != cudaSuccess ||
+              cudaMemcpy(t.type, packed.data(), sizeof(int) * n, cudaMemcpyHostToDevice) !=
+                  cudaSuccess))
+    rc = fail(kCudaError, "engine_set_soft_core: type upload failed");
+  if (rc) {
+    t.release();
+    return rc;
+  }
+  *out = t;
   return kOk;
 }
 
@@ -1422,7 +1442,7 @@ static int engine_forces(snb_engine* e, const float* crd, int step, bool energy,
   prof_mark(e, 1, st);
   const bool do_pme = e->pme.reciprocal && step % e->pme.update_interval == 0;
   const bool groups = e->nl.groups;
-  const int* types = !groups ? e->lj.d_type : (e->soft ? e->d_soft_type : e->d_gtype);
+  const int* types = !groups ? e->lj.d_type : (e->soft ? e->soft_tab.type : e->d_gtype);
   if (e->soft && (!groups || !types))
     return fail(kNotSupported, "soft-core rows: type tables too large");
   if (do_pme)
@@ -1480,9 +1500,9 @@ static int engine_forces(snb_engine* e, const float* crd, int step, bool energy,
     a.bv = e->bv;
     a.blocks_per_sm = e->pair_blocks_per_sm;
     if (e->soft) {
-      a.lj = e->d_soft_a;
+      a.lj = e->soft_tab.a;
       a.n_types = e->soft->nA;
-      a.lj_b = e->d_soft_b;
+      a.lj_b = e->soft_tab.b;
       a.n_types_b = e->soft->nB;
       a.lambda = e->soft->lambda;
       a.alp_A = e->soft->alpha * powf(e->soft->lambda, e->soft->p);
@@ -1845,13 +1865,17 @@ extern "C" int snb_engine_set_soft_core(snb_engine* e, snb_lj_soft* soft) {
       return fail(kNotSupported, "engine_set_soft_core: fixed-point accumulation only");
     if (soft->n != e->n) return fail(kBadInput, "engine_set_soft_core: atom count differs");
   }
-  e->soft = soft;
   if (soft) {
-    e->cluster_form = false;
+    // a failure here leaves the engine with the module it had
     SNB_CUDA_TRY(cudaDeviceSynchronize());  // steps queued with the previous tables
-    const int rc = engine_soft_tables(e, soft);
+    SoftTables t;
+    const int rc = engine_soft_tables(soft, &t);
     if (rc) return rc;
+    e->soft_tab.release();
+    e->soft_tab = t;
+    e->cluster_form = false;
   }
+  e->soft = soft;
   if (soft) {
     const double vol = (double)e->cell.a11 * e->cell.a22 * e->cell.a33;
     e->lrc_energy = soft->lrc / vol;
@@ -2585,9 +2609,7 @@ extern "C" int snb_engine_destroy(snb_engine* e) {
   cudaFree(e->d_prune);
   cudaFree(e->d_lj_tab);
   cudaFree(e->d_gtype);
-  cudaFree(e->d_soft_a);
-  cudaFree(e->d_soft_b);
-  cudaFree(e->d_soft_type);
+  e->soft_tab.release();
   for (void* p : {(void*)e->d_ba, (void*)e->d_bb, (void*)e->d_bk, (void*)e->d_br0,
                   (void*)e->d_aa, (void*)e->d_ab, (void*)e->d_ac, (void*)e->d_ak,
                   (void*)e->d_at0})

@@ -9,6 +9,7 @@ direct Coulomb energies within 2e-6 of their magnitude; the tail term within
 1e-6 relative."""
 
 import ctypes
+import dataclasses
 
 import numpy as np
 import pytest
@@ -105,3 +106,56 @@ def test_engine_soft_core_md_runs(g, soft_box):
         out.append(crd.cpu().numpy())
     assert np.isfinite(out[1]).all()
     assert np.array_equal(out[0], out[1])
+
+
+def _more_types(sc, types):
+    """The same module with unused types behind the used ones in both states."""
+    def grow(t, n):
+        out = np.zeros(types * (types + 1) // 2, np.float32)
+        out[:n * (n + 1) // 2] = t
+        return out
+    return dataclasses.replace(
+        sc, AA=grow(sc.AA, sc.n_types_A), AB=grow(sc.AB, sc.n_types_A), n_types_A=types,
+        BA=grow(sc.BA, sc.n_types_B), BB=grow(sc.BB, sc.n_types_B), n_types_B=types)
+
+
+def test_engine_takes_the_tables_of_the_module_set_last(g, soft_box):
+    """A second module has its own tables: with other row strides the forces
+    stay the same bit for bit, and one whose type tables are too large (80
+    types in both states, 52 KB) has its steps refused whatever was set before
+    it, without touching the forces; the first module, and none, work again
+    after it."""
+    import torch
+    s, sc = soft_box
+    lib = g.capi.load()
+    box = g.Box(s)
+    e = g.engine_create(s, CUTOFF)
+    first, wider, large = (g.soft_create(box, x, CUTOFF, _params(0.5))
+                           for x in (sc, _more_types(sc, 60), _more_types(sc, 80)))
+    crd = g.dev(s.crd.reshape(-1), np.float32)
+
+    def force(module):
+        frc = torch.zeros(3 * s.n, dtype=torch.float32, device="cuda")
+        g.capi.check(lib.snb_engine_set_soft_core(e, module), "set_soft_core")
+        rc = lib.snb_engine_force(e, g.ptr(crd), g.ptr(frc), 0, 0, 0, None, g.stream())
+        torch.cuda.synchronize()
+        return rc, frc.cpu().numpy()
+
+    try:
+        rc, plain = force(None)
+        assert rc == 0
+        rc, want = force(first)
+        assert rc == 0 and not np.array_equal(want, plain)
+        for module in (wider, first):
+            rc, got = force(module)
+            assert rc == 0 and np.array_equal(got, want)
+        rc, got = force(large)
+        assert rc != 0 and not got.any()
+        assert b"type tables too large" in lib.snb_last_error()
+        for module, f in ((first, want), (None, plain), (wider, want)):
+            rc, got = force(module)
+            assert rc == 0 and np.array_equal(got, f)
+    finally:
+        lib.snb_engine_destroy(e)
+        for h in (first, wider, large):
+            lib.snb_lj_soft_destroy(h)
