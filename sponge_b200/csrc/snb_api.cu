@@ -208,6 +208,14 @@ struct snb_engine {
   double prof_ms[7] = {0, 0, 0, 0, 0, 0, 0};
 };
 
+// Forgets the captured step; the next graph step captures again.
+static void drop_graph(snb_engine* e) {
+  if (e->graph_exec) cudaGraphExecDestroy(e->graph_exec);
+  if (e->graph) cudaGraphDestroy(e->graph);
+  e->graph_exec = nullptr;
+  e->graph = nullptr;
+}
+
 static void prof_mark(snb_engine* e, int k, cudaStream_t st) {
   if (e->prof_on) cudaEventRecord(e->prof_ev[k], st);
 }
@@ -1679,11 +1687,7 @@ extern "C" int snb_engine_set_nb14(snb_engine* e, snb_nb14* nb14) {
     }
   }
   e->nb14 = nb14;
-  if (e->graph_exec) {  // the captured step holds the previous set of terms
-    cudaGraphExecDestroy(e->graph_exec);
-    cudaGraphDestroy(e->graph);
-    e->graph_exec = nullptr;
-  }
+  drop_graph(e);  // the captured step holds the previous set of terms
   return kOk;
 }
 
@@ -1792,11 +1796,7 @@ extern "C" int snb_engine_set_settle(snb_engine* e, snb_settle* settle) {
     if (settle->s.n != e->n) return fail(kBadInput, "engine_set_settle: atom count differs");
   }
   e->settle = settle;
-  if (e->graph_exec) {  // the captured step holds the previous integration
-    cudaGraphExecDestroy(e->graph_exec);
-    cudaGraphDestroy(e->graph);
-    e->graph_exec = nullptr;
-  }
+  drop_graph(e);  // the captured step holds the previous integration
   return kOk;
 }
 
@@ -1829,11 +1829,7 @@ extern "C" int snb_engine_update_box(snb_engine* e, snb_boundary boundary) {
     e->lrc_energy = e->lrc_energy_lj;
     e->lrc_virial = e->lrc_virial_lj;
   }
-  if (e->graph_exec) {  // the captured step holds the old box and list arrays
-    cudaGraphExecDestroy(e->graph_exec);
-    cudaGraphDestroy(e->graph);
-    e->graph_exec = nullptr;
-  }
+  drop_graph(e);  // the captured step holds the old box and list arrays
   e->steps_done = 0;  // the next step rebuilds the list, as after Initial
   return kOk;
 }
@@ -1848,12 +1844,7 @@ extern "C" int snb_engine_set_virtual_atoms(snb_engine* e, snb_vatom* vatom) {
       return fail(kBadInput, "engine_set_virtual_atoms: atom count differs");
   }
   e->vatom = vatom;
-  if (e->graph_exec) {  // the captured step holds the previous step shape
-    cudaGraphExecDestroy(e->graph_exec);
-    cudaGraphDestroy(e->graph);
-    e->graph_exec = nullptr;
-    e->graph = nullptr;
-  }
+  drop_graph(e);  // the captured step holds the previous step shape
   return kOk;
 }
 
@@ -1884,11 +1875,7 @@ extern "C" int snb_engine_set_soft_core(snb_engine* e, snb_lj_soft* soft) {
     e->lrc_energy = e->lrc_energy_lj;
     e->lrc_virial = e->lrc_virial_lj;
   }
-  if (e->graph_exec) {  // the captured step holds the previous pair kernel
-    cudaGraphExecDestroy(e->graph_exec);
-    cudaGraphDestroy(e->graph);
-    e->graph_exec = nullptr;
-  }
+  drop_graph(e);  // the captured step holds the previous pair kernel
   return kOk;
 }
 
@@ -1926,12 +1913,7 @@ extern "C" int snb_engine_set_bonded(snb_engine* e, int nb, const int* ba, const
   if (rc) return fail(kCudaError, "engine_set_bonded: upload failed");
   e->nb = nb;
   e->na = na;
-  if (e->graph_exec) {
-    cudaGraphExecDestroy(e->graph_exec);
-    cudaGraphDestroy(e->graph);
-    e->graph_exec = nullptr;
-    e->graph = nullptr;
-  }
+  drop_graph(e);
   return kOk;
 }
 
@@ -2021,11 +2003,7 @@ static int engine_run(snb_engine* e, float* crd, float* vel, const float* invm, 
       if (use_graph && !forced) {
         if (!e->graph_exec || e->g_crd != crd || e->g_vel != vel || e->g_invm != invm ||
             e->g_dt != dt || e->g_stream != st || e->g_vel_wait != e->vel_wait) {
-          if (e->graph_exec) {
-            cudaGraphExecDestroy(e->graph_exec);
-            cudaGraphDestroy(e->graph);
-            e->graph_exec = nullptr;
-          }
+          drop_graph(e);
           SNB_CUDA_TRY(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
           int rc = engine_md_step(e, crd, vel, invm, dt, step, false, st, true);
           cudaGraph_t g = nullptr;
@@ -2084,11 +2062,7 @@ static int engine_run(snb_engine* e, float* crd, float* vel, const float* invm, 
       if (e->opt.nl_throw_error_when_overflow)
         return fail(kOverflow, "neighbor list overflow");
       if (++retries > 8) return fail(kOverflow, "neighbor list overflow persists");
-      if (e->graph_exec) {  // the graph holds the old list pointer
-        cudaGraphExecDestroy(e->graph_exec);
-        cudaGraphDestroy(e->graph);
-        e->graph_exec = nullptr;
-      }
+      drop_graph(e);  // the graph holds the old list pointer
       SNB_CUDA_TRY(cudaMemcpyAsync(crd, e->d_snap_crd, sizeof(float) * 3 * e->n,
                                    cudaMemcpyDeviceToDevice, st));
       SNB_CUDA_TRY(cudaMemcpyAsync(vel, e->d_snap_vel, sizeof(float) * 3 * e->n,
@@ -2364,14 +2338,9 @@ extern "C" int snb_engine_autotune(snb_engine* e, float* crd, float* vel,
   cudaFree(v0);
   cudaEventDestroy(t0);
   cudaEventDestroy(t1);
-  if (rc) return rc;
   e->steps_done = 0;  // the next step rebuilds the list for the restored frame
-  if (e->graph_exec) {  // recapture with the chosen shapes
-    cudaGraphExecDestroy(e->graph_exec);
-    cudaGraphDestroy(e->graph);
-    e->graph_exec = nullptr;
-    e->graph = nullptr;
-  }
+  drop_graph(e);  // recapture with the chosen shapes
+  if (rc) return rc;
   if (h_choice) {
     h_choice[0] = e->pair_unroll;
     h_choice[1] = e->pair_blocks_per_sm;
@@ -2412,12 +2381,7 @@ extern "C" int snb_engine_set_launch_shapes(snb_engine* e, const int* h_choice) 
   e->pme.gather_threads = gt;
   e->pair_warps = w;
   e->pair_stash = sx != 0;
-  if (e->graph_exec) {  // recapture with these shapes
-    cudaGraphExecDestroy(e->graph_exec);
-    cudaGraphDestroy(e->graph);
-    e->graph_exec = nullptr;
-    e->graph = nullptr;
-  }
+  drop_graph(e);  // recapture with these shapes
   return kOk;
 }
 
@@ -2488,12 +2452,7 @@ extern "C" int snb_engine_set_list_form(snb_engine* e, int clusters) {
                 "neighbor list: the cluster form needs one rectangular box of at least "
                 "five cells per axis");
   e->cluster_form = clusters != 0;
-  if (e->graph_exec) {  // the captured step holds the previous list form
-    cudaGraphExecDestroy(e->graph_exec);
-    cudaGraphDestroy(e->graph);
-    e->graph_exec = nullptr;
-    e->graph = nullptr;
-  }
+  drop_graph(e);  // the captured step holds the previous list form
   e->steps_done = 0;
   return kOk;
 }
@@ -2516,12 +2475,7 @@ extern "C" int snb_engine_set_prune_margin(snb_engine* e, float margin) {
       const int one = 1;  // rows kept at another margin are redone
       SNB_CUDA_TRY(cudaMemcpy(e->d_prune + 1, &one, sizeof(int), cudaMemcpyHostToDevice));
     }
-    if (e->graph_exec) {  // the captured step holds the previous choice
-      cudaGraphExecDestroy(e->graph_exec);
-      cudaGraphDestroy(e->graph);
-      e->graph_exec = nullptr;
-      e->graph = nullptr;
-    }
+    drop_graph(e);  // the captured step holds the previous choice
   }
   e->prune_margin = margin;
   return kOk;
@@ -2570,8 +2524,7 @@ extern "C" int snb_engine_stats(snb_engine* e, long long* rebuilds, long long* p
 
 extern "C" int snb_engine_destroy(snb_engine* e) {
   if (!e) return kOk;
-  if (e->graph_exec) cudaGraphExecDestroy(e->graph_exec);
-  if (e->graph) cudaGraphDestroy(e->graph);
+  drop_graph(e);
   for (int k = 0; k < 8; ++k)
     if (e->prof_ev[k]) cudaEventDestroy(e->prof_ev[k]);
   if (e->side) cudaStreamDestroy(e->side);

@@ -271,3 +271,42 @@ def test_own_fft_matches_cufft(g, waters):
     assert g.rel_rms(f1, f0) <= 1e-6
     assert abs(t1[4] - t0[4]) <= 1e-6 * abs(t0[4])
     assert np.all(np.abs(t1[8:14] - t0[8:14]) <= 1e-6 * np.abs(t0[8:14]).max())
+
+
+def test_a_changed_engine_forgets_its_captured_step(g, small_box):
+    """Every call that changes what a step holds drops the captured graph
+    whole: graph_info then has none to count, destroying the engine right
+    after frees nothing twice, and the next graph steps capture anew."""
+    import torch
+    from sponge_b200 import capi, systems
+    s = small_box
+    lib = g.capi.load()
+    e = g.engine_create(s, 8.0)
+    g.engine_set_water_bonded(e, s)
+    crd = g.dev(s.crd.reshape(-1), np.float32)
+    vel = g.dev(s.vel.reshape(-1), np.float32)
+    invm = g.dev((1.0 / s.mass).astype(np.float32))
+    dt = ctypes.c_float(0.5e-3 * systems.TIME_CONVERSION)
+    st = torch.cuda.Stream()
+    sp = ctypes.c_void_p(st.cuda_stream)
+    n = [ctypes.c_int(0) for _ in range(3)]
+    shapes = np.array([4, 0, 8, 256, 16, 0, 0, 0, 0], np.int32)
+    changes = [lambda: lib.snb_engine_set_nb14(e, None),
+               lambda: lib.snb_engine_set_settle(e, None),
+               lambda: lib.snb_engine_set_virtual_atoms(e, None),
+               lambda: lib.snb_engine_set_soft_core(e, None),
+               lambda: lib.snb_engine_set_prune_margin(e, ctypes.c_float(0.6)),
+               lambda: lib.snb_engine_set_launch_shapes(e, shapes.ctypes.data),
+               lambda: lib.snb_engine_update_box(e, capi.boundary(s.cell(), s.rcell()))]
+    try:
+        for k, change in enumerate(changes):
+            with torch.cuda.stream(st):
+                capi.check(lib.snb_engine_md_steps_graph(e, g.ptr(crd), g.ptr(vel), g.ptr(invm),
+                                                         dt, 1 + 3 * k, 3, sp), "md")
+            info = [ctypes.byref(x) for x in n]
+            assert lib.snb_engine_graph_info(e, *info, sp) == 0 and n[0].value > 0
+            assert change() == 0
+            assert lib.snb_engine_graph_info(e, *info, sp) != 0, k
+        assert torch.isfinite(crd).all()
+    finally:
+        lib.snb_engine_destroy(e)
