@@ -477,7 +477,9 @@ int snb_engine_set_launch_shapes(snb_engine* e, const int* h_choice);
 int snb_engine_graph_info(snb_engine* e, int* kernel_nodes,
                           int* library_kernel_nodes, int* rebuild_kernel_nodes,
                           void* stream);
-/* Number of neighbor-list rebuilds so far and current pair count (host sync). */
+/* Number of neighbor-list rebuilds so far and current pair count (host sync).
+ * Where the last build outgrew its rows, this call regrows them, and the next
+ * force or step builds the list again. */
 int snb_engine_stats(snb_engine* e, long long* rebuilds, long long* pairs,
                      void* stream);
 /* snb_pme_spread_wide_tiles of the engine's PME (host sync).  A single-box
@@ -519,7 +521,8 @@ int snb_engine_set_prune_margin(snb_engine* e, float margin);
 int snb_engine_prune_passes(snb_engine* e, int* passes, long long* kept_entries,
                             void* stream);
 /* The engine's current pair set in global ids, lo < hi, in no particular
- * order (as snb_nl_export_pairs; host sync). */
+ * order (as snb_nl_export_pairs; host sync).  Refused after a build that
+ * outgrew its rows, until the next force or step has built them again. */
 int snb_engine_export_pairs(snb_engine* e, int* d_pi, int* d_pj, long long cap,
                             long long* count, void* stream);
 int snb_engine_destroy(snb_engine* e);

@@ -216,6 +216,14 @@ static void drop_graph(snb_engine* e) {
   e->graph = nullptr;
 }
 
+// After a call that may have regrown the list: the captured step holds the old
+// rows, and the next force or step builds the new ones.
+static void engine_list_emptied(snb_engine* e) {
+  if (!e->nl.emptied) return;
+  drop_graph(e);
+  e->steps_done = 0;
+}
+
 static void prof_mark(snb_engine* e, int k, cudaStream_t st) {
   if (e->prof_on) cudaEventRecord(e->prof_ev[k], st);
 }
@@ -2040,6 +2048,7 @@ static int engine_run(snb_engine* e, float* crd, float* vel, const float* invm, 
     }
     bool regrown = false;
     int rc = nl_check_overflow(e->nl, &regrown, st);
+    engine_list_emptied(e);  // a rebuild on the next step, in this call or a later one
     if (rc) return rc;
     if (e->vatom) {
       int bad = 0;
@@ -2062,12 +2071,10 @@ static int engine_run(snb_engine* e, float* crd, float* vel, const float* invm, 
       if (e->opt.nl_throw_error_when_overflow)
         return fail(kOverflow, "neighbor list overflow");
       if (++retries > 8) return fail(kOverflow, "neighbor list overflow persists");
-      drop_graph(e);  // the graph holds the old list pointer
       SNB_CUDA_TRY(cudaMemcpyAsync(crd, e->d_snap_crd, sizeof(float) * 3 * e->n,
                                    cudaMemcpyDeviceToDevice, st));
       SNB_CUDA_TRY(cudaMemcpyAsync(vel, e->d_snap_vel, sizeof(float) * 3 * e->n,
                                    cudaMemcpyDeviceToDevice, st));
-      e->steps_done = 0;  // forces a rebuild on the next step
       continue;
     }
     s += chunk;
@@ -2503,7 +2510,9 @@ extern "C" int snb_engine_list_form(snb_engine* e, int* clusters) {
 extern "C" int snb_engine_export_pairs(snb_engine* e, int* d_pi, int* d_pj, long long cap,
                                        long long* count, void* stream) {
   if (!e || !count) return fail(kBadInput, "engine_export_pairs: null argument");
-  return nl_export_pairs(e->nl, d_pi, d_pj, cap, count, S(stream));
+  const int rc = nl_export_pairs(e->nl, d_pi, d_pj, cap, count, S(stream));
+  engine_list_emptied(e);
+  return rc;
 }
 
 extern "C" int snb_engine_spread_wide_tiles(snb_engine* e, int* count, void* stream) {
@@ -2516,6 +2525,7 @@ extern "C" int snb_engine_stats(snb_engine* e, long long* rebuilds, long long* p
   if (!e) return fail(kBadInput, "engine_stats: null handle");
   bool regrown;
   int rc = nl_check_overflow(e->nl, &regrown, S(stream));
+  engine_list_emptied(e);
   if (rc) return rc;
   if (rebuilds) *rebuilds = e->nl.h_flags[3];
   if (pairs) *pairs = e->nl.last_total;

@@ -161,7 +161,8 @@ struct NeighborList {
   int* h_flags = nullptr;       // pinned mirror
   ScanScratch scan;
   long long last_total = 0;
-  int generation = 0;
+  int generation = 0;          // 0: nothing built, the next update rebuilds
+  bool emptied = false;        // regrown after an overflow and not yet rebuilt
   // Grouped rows (the engine's list): a group is up to kGroupSize sorted
   // atoms of one cell, whose atoms follow a path up and down the cell's four
   // xy quarter columns.  Row g lists the partner atoms with a pair within r_l

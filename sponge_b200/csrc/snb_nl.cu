@@ -1193,7 +1193,7 @@ static void groups_free(NeighborList& nl) {
 
 // Storage of the grouped rows for the current grid and row capacity gcap.
 static int groups_alloc(NeighborList& nl) {
-  const bool pruned = nl.d_gmask != nullptr;
+  const bool pruned = nl.d_prune_ref != nullptr;
   groups_free(nl);
   nl.gcap = (std::max(nl.gcap, 32) + 31) & ~31;
   nl.max_groups = nl.n / kGroupSize + nl.ncell;
@@ -1435,6 +1435,7 @@ int nl_decide(NeighborList& nl, const float* crd_f, int step, int forced,
   const int n = nl.n;
   if (nl.generation == 0) forced = 1;  // nothing built yet
   nl.generation += 1;
+  nl.emptied = false;
   if (forced) {
     nl_need_all(nl, st);
   } else if (nl.refresh_interval <= 0) {
@@ -1463,6 +1464,8 @@ int nl_rebuild(NeighborList& nl, const float* crd_f, const int* atom_local,
                cudaStream_t st) {
   const float3* crd = reinterpret_cast<const float3*>(crd_f);
   const int n = nl.n;
+  if (nl.groups ? !nl.d_gentry : !nl.d_cols)
+    return fail(kCudaError, "neighbor list: no memory for the rows");
   // Excluded-partner sets need global ids equal to the caller's indices.
   int* excl_count = (excl_numbers && !atom_local) ? nl.d_excl_count : nullptr;
   const unsigned char* need = nl.bv.nsys > 0 ? nl.bv.box_need : nullptr;
@@ -1600,37 +1603,38 @@ int nl_check_overflow(NeighborList& nl, bool* regrown, cudaStream_t st) {
                                cudaMemcpyDeviceToHost, st));
   SNB_CUDA_TRY(cudaStreamSynchronize(st));
   nl.last_total = nl.h_flags[kFlagTotal];
-  if (nl.h_flags[kFlagListOverflow] && nl.groups) {
-    const long long need = nl.h_flags[kFlagMaxRow];
-    nl.gcap = std::max((int)std::min<long long>(need + need / 5 + 32, nl.n), nl.gcap + 32);
+  if (!nl.h_flags[kFlagListOverflow]) return kOk;
+  // The larger rows start out empty: whoever asked, the next update rebuilds
+  // them (nl_decide forces what has no generation).
+  const long long need = nl.h_flags[kFlagMaxRow];
+  const int cap = (int)std::min<long long>(need + need / 5 + 32, nl.n);
+  const int row_cap = (std::max(cap, nl.row_cap + 32) + 7) & ~7;
+  if (!nl.groups && ((long long)nl.n + 1) * row_cap > 2147483647LL)
+    return fail(kOverflow, "neighbor list: rows exceed 32-bit offsets");
+  nl.generation = 0;
+  nl.emptied = true;
+  if (nl.groups) {
+    nl.gcap = std::max(cap, nl.gcap + 32);
     int rc = groups_alloc(nl);
     if (rc) return rc;
-    int zero = 0;
-    SNB_CUDA_TRY(cudaMemcpyAsync(nl.d_flags + kFlagListOverflow, &zero, sizeof(int),
-                                 cudaMemcpyHostToDevice, st));
-    SNB_CUDA_TRY(cudaStreamSynchronize(st));
-    *regrown = true;
-    return kOk;
-  }
-  if (nl.h_flags[kFlagListOverflow]) {
-    long long need = nl.h_flags[kFlagMaxRow];
-    int cap = (int)std::min<long long>(need + need / 5 + 32, nl.n);
+  } else {
+    SNB_CUDA_TRY(cudaMemsetAsync(nl.d_row_count, 0, sizeof(int) * nl.n, st));
     SNB_CUDA_TRY(cudaFree(nl.d_cols));
-    nl.row_cap = (std::max(cap, nl.row_cap + 32) + 7) & ~7;
-    nl.cap = (long long)nl.row_cap * nl.n;
-    if (nl.cap + nl.row_cap > 2147483647LL)
-      return fail(kOverflow, "neighbor list: rows exceed 32-bit offsets");
+    nl.d_cols = nullptr;
+    nl.row_cap = row_cap;
+    nl.cap = (long long)row_cap * nl.n;
     SNB_CUDA_TRY(cudaMalloc(&nl.d_cols, sizeof(int) * nl.cap));
     k_row_starts<<<ceil_div(nl.n + 1, 256), 256, 0, st>>>(nl.n, nl.row_cap, nl.d_row_start);
-    int zero = 0;
-    SNB_CUDA_TRY(cudaMemcpyAsync(nl.d_flags + kFlagListOverflow, &zero, sizeof(int),
-                                 cudaMemcpyHostToDevice, st));
-    SNB_CUDA_TRY(cudaStreamSynchronize(st));
-    *regrown = true;
   }
+  int zero = 0;
+  SNB_CUDA_TRY(cudaMemcpyAsync(nl.d_flags + kFlagListOverflow, &zero, sizeof(int),
+                               cudaMemcpyHostToDevice, st));
+  SNB_CUDA_TRY(cudaStreamSynchronize(st));
+  *regrown = true;
   return kOk;
 }
 
+// The pairs of the last build (counted in full where the rows overflowed).
 int nl_total_pairs(NeighborList& nl, long long* total, cudaStream_t st) {
   bool regrown;
   int rc = nl_check_overflow(nl, &regrown, st);
@@ -1641,6 +1645,9 @@ int nl_total_pairs(NeighborList& nl, long long* total, cudaStream_t st) {
 
 // ---------------------------------------------------------------------------
 // Exports.
+static const char* const kEmptied =
+    "neighbor list export: the rows were too short and have been regrown; the next update "
+    "builds them again";
 struct AtomGroupABI {  // layout of the reference's ATOM_GROUP (common.h:177-182)
   int atom_numbers;
   int ghost_numbers;
@@ -1715,6 +1722,7 @@ int nl_export_atom_groups(NeighborList& nl, void* d_groups, int* d_slab,
                           int max_neighbor_numbers, cudaStream_t st) {
   if (nl.groups)
     return fail(kNotSupported, "neighbor list export: ATOM_GROUP rows of grouped rows");
+  if (nl.emptied) return fail(kOverflow, kEmptied);
   const int n = nl.n;
   int* counts = nullptr;
   SNB_CUDA_TRY(cudaMallocAsync(&counts, sizeof(int) * n, st));
@@ -1817,6 +1825,7 @@ int nl_export_pairs(NeighborList& nl, int* d_pi, int* d_pj, long long cap,
   int rc = nl_total_pairs(nl, &total, st);
   if (rc) return rc;
   *count = total;
+  if (nl.emptied) return fail(kOverflow, kEmptied);
   if (total > cap) return fail(kOverflow, "export_pairs: capacity too small");
   if (nl.groups) {
     unsigned long long* next = nullptr;

@@ -42,6 +42,28 @@ def _pairs(g, e):
     return p[np.lexsort((p[:, 1], p[:, 0]))]
 
 
+def _want(oracle, s, cutoff, tol=1e-5):
+    """FP64 forces of the engine's terms over the oracle's pairs."""
+    from sponge_b200 import systems
+    rs, cols = oracle.nl_pairs_system(s, cutoff, 2.0)
+    beta = oracle.get_beta(cutoff, tol)
+    return (oracle.direct_f64(s, cutoff, beta, rs, cols)["frc"] +
+            oracle.excluded_f64(s, beta)["frc"] +
+            oracle.pme_f64(s, (systems.fft_size(s.box),) * 3, beta)["frc"])
+
+
+def _spread_and_packed(waters=1000, factor=1.8):
+    """The same molecules twice in one large box: drawn apart over all of it,
+    and as a dense block in one corner, whose rows outgrow the capacity that
+    the mean density gave."""
+    from sponge_b200 import systems
+    s = systems.water_box(waters, seed=21)
+    o = np.repeat(s.crd[::3], 3, axis=0)
+    apart = (s.crd - o) + o * np.float32(factor)
+    return (dataclasses.replace(s, crd=apart.astype(np.float32), box=s.box * factor),
+            dataclasses.replace(s, box=s.box * factor))
+
+
 def _check(g, oracle, s, cutoff, tol=1e-5):
     import torch
     from sponge_b200 import systems
@@ -120,3 +142,88 @@ def test_many_exclusions_and_types(g, oracle):
                             excl_list=np.concatenate(lists).astype(np.int32))
     s.lj_type[::3] = rng.choice([0, 2, 3], len(s.lj_type[::3]))
     _check(g, oracle, s, 7.0)
+
+
+def _force_of(g, e, crd, n, step, sp=None):
+    import torch
+    frc = torch.zeros(3 * n, dtype=torch.float32, device="cuda")
+    g.capi.check(g.capi.load().snb_engine_force(e, g.ptr(crd), g.ptr(frc), step, 0, 0, None,
+                                                sp or g.stream()), "engine_force")
+    torch.cuda.synchronize()
+    return frc.cpu().numpy().reshape(n, 3)
+
+
+@pytest.mark.parametrize("ask", ["stats", "export"])
+def test_overflow_seen_between_steps_rebuilds(g, oracle, ask):
+    """A later rebuild outgrows the rows and a call between steps is the first
+    to see it: the count is the new frame's, the export is refused, and the
+    next force on the same coordinates and the next graph steps (captured
+    before with the old rows) build the list again."""
+    import torch
+    from sponge_b200 import systems
+    spread, packed = _spread_and_packed()
+    lib = g.capi.load()
+    e = g.engine_create(spread, 7.0)
+    g.engine_set_water_bonded(e, spread)
+    state = g.dev(spread.crd.reshape(-1), np.float32)
+    vel = torch.zeros_like(state)
+    invm = g.dev((1.0 / spread.mass).astype(np.float32))
+    dense = g.dev(packed.crd.reshape(-1), np.float32)
+    dt = ctypes.c_float(1e-4 * systems.TIME_CONVERSION)
+    st = torch.cuda.Stream()
+    sp = ctypes.c_void_p(st.cuda_stream)
+    pi = torch.empty(1, dtype=torch.int32, device="cuda")
+    count = ctypes.c_longlong(0)
+
+    def steps(first):
+        g.capi.check(lib.snb_engine_md_steps_graph(e, g.ptr(state), g.ptr(vel), g.ptr(invm), dt,
+                                                   first, 3, sp), "md")
+        st.synchronize()
+
+    try:
+        torch.cuda.synchronize()
+        steps(1)
+        _force_of(g, e, dense, packed.n, 1, sp)
+        if ask == "stats":
+            g.capi.check(lib.snb_engine_stats(e, None, ctypes.byref(count), sp), "stats")
+        else:
+            assert lib.snb_engine_export_pairs(e, g.ptr(pi), g.ptr(pi), 1, ctypes.byref(count),
+                                               sp) != 0
+        rs, cols = oracle.nl_pairs_system(packed, 7.0, 2.0)
+        assert count.value == len(cols)
+        assert lib.snb_engine_export_pairs(e, g.ptr(pi), g.ptr(pi), count.value,
+                                           ctypes.byref(count), sp) != 0
+        assert b"builds them again" in lib.snb_last_error()
+        got = _force_of(g, e, dense, packed.n, 1, sp)
+        assert g.rel_rms(got, _want(oracle, packed, 7.0)) <= 1e-5
+        assert np.array_equal(_pairs(g, e), g.csr_to_pairs(rs, cols))
+        before = state.clone()
+        steps(4)
+        assert torch.isfinite(state).all() and not torch.equal(state, before)
+    finally:
+        lib.snb_engine_destroy(e)
+
+
+def test_module_list_overflow_between_updates_rebuilds(g, oracle):
+    """The modules' rows likewise: emptied by the count that found them too
+    short, refused to the export, built by the next conditional update."""
+    spread, packed = _spread_and_packed()
+    lib = g.capi.load()
+    box, dense = g.Box(spread), g.Box(packed)
+    h = g.make_nl(box, 7.0, 2.0)
+    import torch
+    pi = torch.empty(1, dtype=torch.int32, device="cuda")
+    count = ctypes.c_longlong(0)
+    try:
+        g.nl_update(h, box)
+        g.nl_update(h, dense)
+        g.capi.check(lib.snb_nl_pair_count(h, ctypes.byref(count), g.stream()), "count")
+        rs, cols = oracle.nl_pairs_system(packed, 7.0, 2.0)
+        assert count.value == len(cols)
+        assert lib.snb_nl_export_pairs(h, g.ptr(pi), g.ptr(pi), count.value,
+                                       ctypes.byref(count), g.stream()) != 0
+        assert b"builds them again" in lib.snb_last_error()
+        g.nl_update(h, dense, forced=0)
+        assert np.array_equal(g.nl_pairs(h), g.csr_to_pairs(rs, cols))
+    finally:
+        lib.snb_nl_destroy(h)
