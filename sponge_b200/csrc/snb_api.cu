@@ -470,7 +470,7 @@ extern "C" int snb_lj_create(const snb_options* opt, int atom_numbers,
   SNB_CUDA_TRY(cudaMalloc(&h->d_pos, sizeof(float4) * atom_numbers));
   SNB_CUDA_TRY(cudaMalloc(&h->d_type_sorted, sizeof(int) * atom_numbers));
   SNB_CUDA_TRY(cudaMalloc(&h->d_lj_energy, sizeof(float) * atom_numbers));
-  SNB_CUDA_TRY(cudaMemset(h->d_lj_energy, 0, sizeof(float) * atom_numbers));
+  SNB_CUDA_TRY(clear_now(h->d_lj_energy, sizeof(float) * atom_numbers));
   SNB_CUDA_TRY(cudaMalloc(&h->d_sum, sizeof(double)));
   *out = h;
   return kOk;
@@ -747,9 +747,9 @@ extern "C" int snb_lj_soft_create(const snb_options* opt, int n, int nA, int nB,
   SNB_CUDA_TRY(cudaMalloc(&h->d_lj_energy, sizeof(float) * n));
   SNB_CUDA_TRY(cudaMalloc(&h->d_inter, sizeof(float) * n));
   SNB_CUDA_TRY(cudaMalloc(&h->d_intra, sizeof(float) * n));
-  SNB_CUDA_TRY(cudaMemset(h->d_lj_energy, 0, sizeof(float) * n));
-  SNB_CUDA_TRY(cudaMemset(h->d_inter, 0, sizeof(float) * n));
-  SNB_CUDA_TRY(cudaMemset(h->d_intra, 0, sizeof(float) * n));
+  SNB_CUDA_TRY(clear_now(h->d_lj_energy, sizeof(float) * n));
+  SNB_CUDA_TRY(clear_now(h->d_inter, sizeof(float) * n));
+  SNB_CUDA_TRY(clear_now(h->d_intra, sizeof(float) * n));
   SNB_CUDA_TRY(cudaMalloc(&h->d_dudl, sizeof(long long) * 2));
   int rc = acc_init(h->acc, n);
   if (rc) return rc;
@@ -1191,12 +1191,12 @@ static int engine_finish_create(snb_engine* e, int n, int n_types, const int* h_
       SNB_CUDA_TRY(cudaMemcpy(e->d_excl_list, h_el, sizeof(int) * n_excl,
                               cudaMemcpyHostToDevice));
   } else {
-    SNB_CUDA_TRY(cudaMemset(e->d_excl_start, 0, sizeof(int) * n));
-    SNB_CUDA_TRY(cudaMemset(e->d_excl_numbers, 0, sizeof(int) * n));
+    SNB_CUDA_TRY(clear_now(e->d_excl_start, sizeof(int) * n));
+    SNB_CUDA_TRY(clear_now(e->d_excl_numbers, sizeof(int) * n));
   }
   SNB_CUDA_TRY(cudaMalloc(&e->d_isum, sizeof(long long) * 9));
   SNB_CUDA_TRY(cudaMalloc(&e->d_bonded_e, sizeof(long long)));
-  SNB_CUDA_TRY(cudaMemset(e->d_bonded_e, 0, sizeof(long long)));
+  SNB_CUDA_TRY(clear_now(e->d_bonded_e, sizeof(long long)));
   SNB_CUDA_TRY(cudaMalloc(&e->d_totals_scratch, sizeof(double) * 16));
   SNB_CUDA_TRY(cudaMalloc(&e->d_snap_crd, sizeof(float) * 3 * n));
   SNB_CUDA_TRY(cudaMalloc(&e->d_snap_vel, sizeof(float) * 3 * n));
@@ -1215,6 +1215,7 @@ static int engine_finish_create(snb_engine* e, int n, int n_types, const int* h_
   SNB_CUDA_TRY(cudaEventCreateWithFlags(&e->ev_crd_in, cudaEventDisableTiming));
   SNB_CUDA_TRY(cudaEventCreateWithFlags(&e->ev_vel_in, cudaEventDisableTiming));
   SNB_CUDA_TRY(cudaEventRecord(e->ev_vel_in, e->io));  // a completed record
+  SNB_CUDA_TRY(cudaStreamSynchronize(nullptr));  // the copies above, for any stream
   return kOk;
 }
 
@@ -1351,7 +1352,7 @@ extern "C" int snb_batch_create(const snb_options* opt, int n_systems,
         cudaMemcpy(e->d_cell_sys, cell_sys.data(), sizeof(int) * cell_sys.size(),
                    cudaMemcpyHostToDevice) != cudaSuccess ||
         cudaMalloc(&e->d_box_need, n_systems) != cudaSuccess ||
-        cudaMemset(e->d_box_need, 0, n_systems) != cudaSuccess)
+        clear_now(e->d_box_need, n_systems) != cudaSuccess)
       rc = fail(kCudaError, "batch_create: per-system rebuild tables failed");
   }
   if (!rc) {
@@ -1633,7 +1634,7 @@ extern "C" int snb_nb14_create(int atom_numbers, int nb14_numbers, const int* h_
   if (!rc) rc = acc_init(h->acc, atom_numbers);
   if (!rc) {
     cudaError_t ce = cudaMalloc(&h->d_sums, sizeof(long long) * 2);
-    if (ce == cudaSuccess) ce = cudaMemset(h->d_sums, 0, sizeof(long long) * 2);
+    if (ce == cudaSuccess) ce = clear_now(h->d_sums, sizeof(long long) * 2);
     if (ce != cudaSuccess) rc = fail(kCudaError, cudaGetErrorString(ce));
   }
   if (rc) {
@@ -1691,7 +1692,7 @@ extern "C" int snb_engine_set_nb14(snb_engine* e, snb_nb14* nb14) {
     if (nb14->n != e->n) return fail(kBadInput, "engine_set_nb14: atom count differs");
     if (!e->d_nb14_sums) {
       SNB_CUDA_TRY(cudaMalloc(&e->d_nb14_sums, sizeof(long long) * 2));
-      SNB_CUDA_TRY(cudaMemset(e->d_nb14_sums, 0, sizeof(long long) * 2));
+      SNB_CUDA_TRY(clear_now(e->d_nb14_sums, sizeof(long long) * 2));
     }
   }
   e->nb14 = nb14;
@@ -2469,8 +2470,9 @@ extern "C" int snb_engine_set_prune_margin(snb_engine* e, float margin) {
   if (!(margin >= 0.f) || margin > 100.f)
     return fail(kBadInput, "engine_set_prune_margin: margin must be in [0, 100] A");
   if (margin > 0.f) {
-    int rc = nl_enable_prune(e->nl);
+    int rc = nl_enable_prune(e->nl, nullptr);
     if (rc) return rc;
+    SNB_CUDA_TRY(cudaStreamSynchronize(nullptr));
     if (!e->d_prune) {
       SNB_CUDA_TRY(cudaMalloc(&e->d_prune, sizeof(int) * 4));
       const int init[4] = {0, 1, -1, 0};  // the first step prunes

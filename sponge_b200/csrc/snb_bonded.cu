@@ -153,7 +153,7 @@ static int terms_init(TermList& t, int atom_numbers, int m, const int* a, const 
   if (!rc) rc = acc_init(t.acc, atom_numbers);
   if (!rc) {
     SNB_CUDA_TRY(cudaMalloc(&t.d_sum, sizeof(long long)));
-    SNB_CUDA_TRY(cudaMemset(t.d_sum, 0, sizeof(long long)));
+    SNB_CUDA_TRY(clear_now(t.d_sum, sizeof(long long)));
   }
   return rc;
 }

@@ -36,6 +36,14 @@ int fail(int code, const std::string& msg);
                          std::string(#expr) + ": " + cudaGetErrorString(e_)); \
   } while (0)
 
+// Clears device memory before it returns.  cudaMemset alone is queued on the
+// legacy default stream, which the callers' non-blocking streams do not wait
+// for.
+inline cudaError_t clear_now(void* p, size_t bytes) {
+  const cudaError_t e = cudaMemset(p, 0, bytes);
+  return e != cudaSuccess ? e : cudaStreamSynchronize(nullptr);
+}
+
 // Scratch for the device-wide exclusive scan (3-phase).
 struct ScanScratch {
   int* block_sums = nullptr;
@@ -194,8 +202,9 @@ int nl_init_batch(NeighborList& nl, int n, float cutoff, float skin,
                   std::vector<SysGeom>& sys, int refresh_interval, float skin_permit,
                   int max_neighbor_numbers, bool groups = false);
 void nl_free(NeighborList& nl);
-// Allocates what the pruned rows need (the kept-atom bytes of grouped rows).
-int nl_enable_prune(NeighborList& nl);
+// Allocates what the pruned rows need (the kept-atom bytes of grouped rows,
+// cleared on st).
+int nl_enable_prune(NeighborList& nl, cudaStream_t st);
 // Entries of the batches that the last prune pass kept (host sync).
 int nl_kept_entries(NeighborList& nl, long long* kept, cudaStream_t st);
 // Update as NEIGHBOR_LIST::Update (neighbor_list.cpp:974-1025): forced, or

@@ -1191,8 +1191,9 @@ static void groups_free(NeighborList& nl) {
   nl.d_gmask = nullptr;
 }
 
-// Storage of the grouped rows for the current grid and row capacity gcap.
-static int groups_alloc(NeighborList& nl) {
+// Storage of the grouped rows for the current grid and row capacity gcap, with
+// every row empty for work that is queued on st afterwards.
+static int groups_alloc(NeighborList& nl, cudaStream_t st) {
   const bool pruned = nl.d_prune_ref != nullptr;
   groups_free(nl);
   nl.gcap = (std::max(nl.gcap, 32) + 31) & ~31;
@@ -1200,13 +1201,13 @@ static int groups_alloc(NeighborList& nl) {
   const size_t G = nl.max_groups;
   SNB_CUDA_TRY(cudaMalloc(&nl.d_atom_key, sizeof(int) * nl.n));
   SNB_CUDA_TRY(cudaMalloc(&nl.d_group, sizeof(int2) * G));
-  SNB_CUDA_TRY(cudaMemset(nl.d_group, 0, sizeof(int2) * G));
+  SNB_CUDA_TRY(cudaMemsetAsync(nl.d_group, 0, sizeof(int2) * G, st));
   SNB_CUDA_TRY(cudaMalloc(&nl.d_grow_count, sizeof(int) * G));
-  SNB_CUDA_TRY(cudaMemset(nl.d_grow_count, 0, sizeof(int) * G));
+  SNB_CUDA_TRY(cudaMemsetAsync(nl.d_grow_count, 0, sizeof(int) * G, st));
   SNB_CUDA_TRY(cudaMalloc(&nl.d_gpairs, sizeof(int) * G));
-  SNB_CUDA_TRY(cudaMemset(nl.d_gpairs, 0, sizeof(int) * G));
+  SNB_CUDA_TRY(cudaMemsetAsync(nl.d_gpairs, 0, sizeof(int) * G, st));
   SNB_CUDA_TRY(cudaMalloc(&nl.d_gentry, sizeof(unsigned) * G * nl.gcap));
-  if (pruned) return nl_enable_prune(nl);
+  if (pruned) return nl_enable_prune(nl, st);
   return kOk;
 }
 
@@ -1235,7 +1236,7 @@ static int nl_alloc(NeighborList& nl, int n, long long initial_capacity,
   SNB_CUDA_TRY(cudaMalloc(&nl.d_pos, sizeof(float4) * n));
   SNB_CUDA_TRY(cudaMalloc(&nl.d_old_crd, sizeof(float3) * n));
   SNB_CUDA_TRY(cudaMalloc(&nl.d_flags, sizeof(int) * kNumFlags));
-  SNB_CUDA_TRY(cudaMemset(nl.d_flags, 0, sizeof(int) * kNumFlags));
+  SNB_CUDA_TRY(clear_now(nl.d_flags, sizeof(int) * kNumFlags));
   SNB_CUDA_TRY(cudaMallocHost(&nl.h_flags, sizeof(int) * kNumFlags));
   SNB_CUDA_TRY(cudaMalloc(&nl.d_unsorted, sizeof(int) * n));
   SNB_CUDA_TRY(cudaMalloc(&nl.d_sorted_cell, sizeof(int) * n));
@@ -1248,8 +1249,8 @@ static int nl_alloc(NeighborList& nl, int n, long long initial_capacity,
                             cudaMemcpyHostToDevice));
     SNB_CUDA_TRY(cudaMemcpy(nl.d_global, iota.data(), sizeof(int) * n,
                             cudaMemcpyHostToDevice));
-    SNB_CUDA_TRY(cudaMemset(nl.d_sorted_cell, 0, sizeof(int) * n));
-    SNB_CUDA_TRY(cudaMemset(nl.d_pos, 0, sizeof(float4) * n));
+    SNB_CUDA_TRY(clear_now(nl.d_sorted_cell, sizeof(int) * n));
+    SNB_CUDA_TRY(clear_now(nl.d_pos, sizeof(float4) * n));
   }
   if (groups && n < kGroupMaxAtoms) {
     nl.groups = true;
@@ -1257,13 +1258,15 @@ static int nl_alloc(NeighborList& nl, int n, long long initial_capacity,
     const double rl = sqrt((double)nl.rl2), s = (rl + 2.0) / rl;
     const double mean = max_per_atom * s * s * s;
     nl.gcap = (int)std::min<double>((all_balanced ? 1.4 : 2.4) * mean + 64.0, n);
-    const int rc = groups_alloc(nl);
-    return rc ? rc : scan_reserve(nl.scan, std::max(nl.ncell, n));
+    const int rc = groups_alloc(nl, nullptr);
+    if (rc) return rc;
+    SNB_CUDA_TRY(cudaStreamSynchronize(nullptr));
+    return scan_reserve(nl.scan, std::max(nl.ncell, n));
   }
   SNB_CUDA_TRY(cudaMalloc(&nl.d_row_count, sizeof(int) * n));
   SNB_CUDA_TRY(cudaMalloc(&nl.d_row_start, sizeof(int) * (n + 1)));
-  SNB_CUDA_TRY(cudaMemset(nl.d_row_count, 0, sizeof(int) * n));
-  SNB_CUDA_TRY(cudaMemset(nl.d_row_start, 0, sizeof(int) * (n + 1)));
+  SNB_CUDA_TRY(clear_now(nl.d_row_count, sizeof(int) * n));
+  SNB_CUDA_TRY(clear_now(nl.d_row_start, sizeof(int) * (n + 1)));
   // Row capacity: 1.5x (2.5x where cell pairs are owned by index, which
   // balances rows less well) the mean half-sphere count plus a margin;
   // regrown on overflow by nl_check_overflow.
@@ -1278,17 +1281,18 @@ static int nl_alloc(NeighborList& nl, int n, long long initial_capacity,
   SNB_CUDA_TRY(cudaMalloc(&nl.d_cols, sizeof(int) * nl.cap));
   k_row_starts<<<ceil_div(n + 1, 256), 256>>>(n, nl.row_cap, nl.d_row_start);
   SNB_CUDA_TRY(cudaGetLastError());
+  SNB_CUDA_TRY(cudaStreamSynchronize(nullptr));
   return scan_reserve(nl.scan, std::max(nl.ncell, n));
 }
 
 // The pruned rows' storage (contents written by the pair kernel's prune
 // passes).
-int nl_enable_prune(NeighborList& nl) {
+int nl_enable_prune(NeighborList& nl, cudaStream_t st) {
   if (!nl.d_prune_ref) SNB_CUDA_TRY(cudaMalloc(&nl.d_prune_ref, sizeof(float4) * nl.n));
   if (nl.groups && !nl.d_gmask) {
     const size_t bytes = (size_t)nl.max_groups * (nl.gcap / 32);
     SNB_CUDA_TRY(cudaMalloc(&nl.d_gmask, bytes));
-    SNB_CUDA_TRY(cudaMemset(nl.d_gmask, 0, bytes));
+    SNB_CUDA_TRY(cudaMemsetAsync(nl.d_gmask, 0, bytes, st));
   }
   return kOk;
 }
@@ -1388,7 +1392,8 @@ int nl_regrid(NeighborList& nl, const float* cell6) {
   nl.generation = 0;  // the next update rebuilds
   if (nl.groups && nl.max_groups != nl.n / kGroupSize + nl.ncell) {
     SNB_CUDA_TRY(cudaDeviceSynchronize());
-    return groups_alloc(nl);
+    if ((rc = groups_alloc(nl, nullptr))) return rc;
+    SNB_CUDA_TRY(cudaStreamSynchronize(nullptr));
   }
   return kOk;
 }
@@ -1615,7 +1620,7 @@ int nl_check_overflow(NeighborList& nl, bool* regrown, cudaStream_t st) {
   nl.emptied = true;
   if (nl.groups) {
     nl.gcap = std::max(cap, nl.gcap + 32);
-    int rc = groups_alloc(nl);
+    int rc = groups_alloc(nl, st);
     if (rc) return rc;
   } else {
     SNB_CUDA_TRY(cudaMemsetAsync(nl.d_row_count, 0, sizeof(int) * nl.n, st));

@@ -1301,9 +1301,9 @@ int pme_init(PME& p, int n, const float* cell6, const float* box_length3,
   SNB_CUDA_TRY(cudaMalloc(&p.d_Q, sizeof(float) * p.nall));
   SNB_CUDA_TRY(cudaMalloc(&p.d_FQ, sizeof(cufftComplex) * p.nfft));
   SNB_CUDA_TRY(cudaMalloc(&p.d_phi, sizeof(float) * p.nall));
-  SNB_CUDA_TRY(cudaMemset(p.d_phi, 0, sizeof(float) * p.nall));
+  SNB_CUDA_TRY(clear_now(p.d_phi, sizeof(float) * p.nall));
   SNB_CUDA_TRY(cudaMalloc(&p.d_tile_count, sizeof(int) * p.ntiles));
-  SNB_CUDA_TRY(cudaMemset(p.d_tile_count, 0, sizeof(int) * p.ntiles));
+  SNB_CUDA_TRY(clear_now(p.d_tile_count, sizeof(int) * p.ntiles));
   SNB_CUDA_TRY(cudaMalloc(&p.d_tile_start, sizeof(int) * (p.ntiles + 1)));
   SNB_CUDA_TRY(cudaMalloc(&p.d_atom_tile, sizeof(int) * n));
   SNB_CUDA_TRY(cudaMalloc(&p.d_atom_slot, sizeof(int) * n));
@@ -1314,9 +1314,9 @@ int pme_init(PME& p, int n, const float* cell6, const float* box_length3,
   p.partial_blocks = std::min(ceil_div(p.nfft, kSpecBlock), 148 * 8);
   SNB_CUDA_TRY(cudaMalloc(&p.d_partial, sizeof(double) * 8 * p.partial_blocks));
   SNB_CUDA_TRY(cudaMalloc(&p.d_sums, sizeof(double) * 8));
-  SNB_CUDA_TRY(cudaMemset(p.d_sums, 0, sizeof(double) * 8));
+  SNB_CUDA_TRY(clear_now(p.d_sums, sizeof(double) * 8));
   SNB_CUDA_TRY(cudaMalloc(&p.d_wide_tiles, sizeof(int)));
-  SNB_CUDA_TRY(cudaMemset(p.d_wide_tiles, 0, sizeof(int)));
+  SNB_CUDA_TRY(clear_now(p.d_wide_tiles, sizeof(int)));
   if (scan_reserve(p.scan, p.ntiles)) return kCudaError;
   if (cufftPlan3d(&p.plan_r2c, p.K[0], p.K[1], p.K[2], CUFFT_R2C) != CUFFT_SUCCESS ||
       cufftPlan3d(&p.plan_c2r, p.K[0], p.K[1], p.K[2], CUFFT_C2R) != CUFFT_SUCCESS)
@@ -1337,12 +1337,12 @@ int pme_set_spread_shape(PME& p, int T, int W) {
   if (T == 0) {
     if (!p.d_Q64) {
       SNB_CUDA_TRY(cudaMalloc(&p.d_Q64, sizeof(long long) * (size_t)p.nall));
-      SNB_CUDA_TRY(cudaMemset(p.d_Q64, 0, sizeof(long long) * (size_t)p.nall));
+      SNB_CUDA_TRY(clear_now(p.d_Q64, sizeof(long long) * (size_t)p.nall));
     }
     if (!p.spread_atomic) {
       // the tile counts restart from zero when the tiles come back
       SNB_CUDA_TRY(cudaDeviceSynchronize());
-      SNB_CUDA_TRY(cudaMemset(p.d_tile_count, 0, sizeof(int) * p.ntiles));
+      SNB_CUDA_TRY(clear_now(p.d_tile_count, sizeof(int) * p.ntiles));
     }
     p.spread_atomic = true;
     return kOk;
@@ -1368,7 +1368,7 @@ int pme_set_spread_shape(PME& p, int T, int W) {
   cudaFree(p.d_tile_count);
   cudaFree(p.d_tile_start);
   SNB_CUDA_TRY(cudaMalloc(&p.d_tile_count, sizeof(int) * ntiles));
-  SNB_CUDA_TRY(cudaMemset(p.d_tile_count, 0, sizeof(int) * ntiles));
+  SNB_CUDA_TRY(clear_now(p.d_tile_count, sizeof(int) * ntiles));
   SNB_CUDA_TRY(cudaMalloc(&p.d_tile_start, sizeof(int) * (ntiles + 1)));
   p.T = T;
   p.ntiles = ntiles;
@@ -1580,13 +1580,13 @@ int pme_init_batch(PME& p, int n, std::vector<SysGeom>& sys, float cutoff,
   SNB_CUDA_TRY(cudaMemcpy(p.d_sys_block_begin, block_begin.data(), sizeof(int) * (nsys + 1),
                           cudaMemcpyHostToDevice));
   SNB_CUDA_TRY(cudaMalloc(&p.d_sys_sums, sizeof(double) * 8 * nsys));
-  SNB_CUDA_TRY(cudaMemset(p.d_sys_sums, 0, sizeof(double) * 8 * nsys));
+  SNB_CUDA_TRY(clear_now(p.d_sys_sums, sizeof(double) * 8 * nsys));
   SNB_CUDA_TRY(cudaMalloc(&p.d_Q, sizeof(float) * p.nall));
   SNB_CUDA_TRY(cudaMalloc(&p.d_FQ, sizeof(cufftComplex) * p.nfft));
   SNB_CUDA_TRY(cudaMalloc(&p.d_phi, sizeof(float) * p.nall));
-  SNB_CUDA_TRY(cudaMemset(p.d_phi, 0, sizeof(float) * p.nall));
+  SNB_CUDA_TRY(clear_now(p.d_phi, sizeof(float) * p.nall));
   SNB_CUDA_TRY(cudaMalloc(&p.d_tile_count, sizeof(int) * p.ntiles));
-  SNB_CUDA_TRY(cudaMemset(p.d_tile_count, 0, sizeof(int) * p.ntiles));
+  SNB_CUDA_TRY(clear_now(p.d_tile_count, sizeof(int) * p.ntiles));
   SNB_CUDA_TRY(cudaMalloc(&p.d_tile_start, sizeof(int) * (p.ntiles + 1)));
   SNB_CUDA_TRY(cudaMalloc(&p.d_atom_tile, sizeof(int) * n));
   SNB_CUDA_TRY(cudaMalloc(&p.d_atom_slot, sizeof(int) * n));
@@ -1597,9 +1597,9 @@ int pme_init_batch(PME& p, int n, std::vector<SysGeom>& sys, float cutoff,
   p.partial_blocks = p.spec_blocks;
   SNB_CUDA_TRY(cudaMalloc(&p.d_partial, sizeof(double) * 8 * p.partial_blocks));
   SNB_CUDA_TRY(cudaMalloc(&p.d_sums, sizeof(double) * 8));
-  SNB_CUDA_TRY(cudaMemset(p.d_sums, 0, sizeof(double) * 8));
+  SNB_CUDA_TRY(clear_now(p.d_sums, sizeof(double) * 8));
   SNB_CUDA_TRY(cudaMalloc(&p.d_wide_tiles, sizeof(int)));
-  SNB_CUDA_TRY(cudaMemset(p.d_wide_tiles, 0, sizeof(int)));
+  SNB_CUDA_TRY(clear_now(p.d_wide_tiles, sizeof(int)));
   if (scan_reserve(p.scan, p.ntiles)) return kCudaError;
   p.h_sys = sys;
   for (auto& fg : p.groups) {

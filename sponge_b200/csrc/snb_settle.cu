@@ -335,10 +335,10 @@ int settle_init(Settle& s, int n, int m, const int* ai, const int* aj, const flo
   SNB_CUDA_TRY(cudaMalloc(&s.d_last_ab, sizeof(float3) * kp));
   SNB_CUDA_TRY(cudaMalloc(&s.d_vir, sizeof(long long) * 6));
   SNB_CUDA_TRY(cudaMalloc(&s.d_err, sizeof(int)));
-  SNB_CUDA_TRY(cudaMemset(s.d_err, 0, sizeof(int)));
-  SNB_CUDA_TRY(cudaMemset(s.d_last_ba, 0, sizeof(float3) * kt));
-  SNB_CUDA_TRY(cudaMemset(s.d_last_ca, 0, sizeof(float3) * kt));
-  SNB_CUDA_TRY(cudaMemset(s.d_last_ab, 0, sizeof(float3) * kp));
+  SNB_CUDA_TRY(clear_now(s.d_err, sizeof(int)));
+  SNB_CUDA_TRY(clear_now(s.d_last_ba, sizeof(float3) * kt));
+  SNB_CUDA_TRY(clear_now(s.d_last_ca, sizeof(float3) * kt));
+  SNB_CUDA_TRY(clear_now(s.d_last_ab, sizeof(float3) * kp));
   if (s.nt)
     SNB_CUDA_TRY(cudaMemcpy(s.d_tri, tri.data(), sizeof(SettleTri) * s.nt,
                             cudaMemcpyHostToDevice));

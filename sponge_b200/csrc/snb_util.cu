@@ -161,14 +161,14 @@ int acc_init(Accumulators& a, int n, bool by_atom) {
   SNB_CUDA_TRY(cudaMalloc(&a.d_fv, sizeof(float) * 6 * N));
   SNB_CUDA_TRY(cudaMalloc(&a.d_eaux, sizeof(long long) * 2 * N));
   SNB_CUDA_TRY(cudaMalloc(&a.d_feaux, sizeof(float) * 2 * N));
-  SNB_CUDA_TRY(cudaMemset(a.d_eaux, 0, sizeof(long long) * 2 * N));
-  SNB_CUDA_TRY(cudaMemset(a.d_feaux, 0, sizeof(float) * 2 * N));
-  SNB_CUDA_TRY(cudaMemset(a.d_f, 0, sizeof(long long) * a.f_len));
-  SNB_CUDA_TRY(cudaMemset(a.d_e, 0, sizeof(long long) * 3 * N));
-  SNB_CUDA_TRY(cudaMemset(a.d_v, 0, sizeof(long long) * 6 * N));
-  SNB_CUDA_TRY(cudaMemset(a.d_ff, 0, sizeof(float) * 3 * N));
-  SNB_CUDA_TRY(cudaMemset(a.d_fe, 0, sizeof(float) * 3 * N));
-  SNB_CUDA_TRY(cudaMemset(a.d_fv, 0, sizeof(float) * 6 * N));
+  SNB_CUDA_TRY(clear_now(a.d_eaux, sizeof(long long) * 2 * N));
+  SNB_CUDA_TRY(clear_now(a.d_feaux, sizeof(float) * 2 * N));
+  SNB_CUDA_TRY(clear_now(a.d_f, sizeof(long long) * a.f_len));
+  SNB_CUDA_TRY(clear_now(a.d_e, sizeof(long long) * 3 * N));
+  SNB_CUDA_TRY(clear_now(a.d_v, sizeof(long long) * 6 * N));
+  SNB_CUDA_TRY(clear_now(a.d_ff, sizeof(float) * 3 * N));
+  SNB_CUDA_TRY(clear_now(a.d_fe, sizeof(float) * 3 * N));
+  SNB_CUDA_TRY(clear_now(a.d_fv, sizeof(float) * 6 * N));
   return kOk;
 }
 

@@ -322,7 +322,7 @@ extern "C" int snb_vatom_create(int atom_numbers, int record_numbers, const int*
   if (ce == cudaSuccess && m > 0)
     ce = cudaMemcpy(h->d_rec, recs.data(), sizeof(VRecord) * m, cudaMemcpyHostToDevice);
   if (ce == cudaSuccess) ce = cudaMalloc(&h->d_err, sizeof(int));
-  if (ce == cudaSuccess) ce = cudaMemset(h->d_err, 0, sizeof(int));
+  if (ce == cudaSuccess) ce = clear_now(h->d_err, sizeof(int));
   if (ce != cudaSuccess) {
     cudaFree(h->d_rec);
     cudaFree(h->d_err);

@@ -227,3 +227,47 @@ def test_module_list_overflow_between_updates_rebuilds(g, oracle):
         assert np.array_equal(g.nl_pairs(h), g.csr_to_pairs(rs, cols))
     finally:
         lib.snb_nl_destroy(h)
+
+
+def test_regrown_rows_beside_default_stream_work(g, oracle):
+    """Rows regrown in the first build, and the pruned rows' bytes made by a
+    new margin, while the legacy default stream is busy: a non-blocking stream
+    does not wait for that one, so clears left on it could land after the
+    rebuild's or the prune pass's writes."""
+    import torch
+    from sponge_b200 import systems
+    spread, packed = _spread_and_packed()
+    lib = g.capi.load()
+    e = g.engine_create(spread, 7.0)
+    dense = g.dev(packed.crd.reshape(-1), np.float32)
+    vel = torch.zeros_like(dense)
+    invm = g.dev((1.0 / packed.mass).astype(np.float32))
+    dt = ctypes.c_float(1e-4 * systems.TIME_CONVERSION)
+    st = torch.cuda.Stream()
+    sp = ctypes.c_void_p(st.cuda_stream)
+    frc = torch.zeros(3 * packed.n, dtype=torch.float32, device="cuda")
+    want = _want(oracle, packed, 7.0)
+    try:
+        for _ in range(2):
+            torch.cuda.synchronize()
+            frc.zero_()
+            torch.cuda._sleep(20_000_000)  # about 10 ms
+            st.wait_stream(torch.cuda.default_stream())
+            torch.cuda._sleep(20_000_000)
+            g.capi.check(lib.snb_engine_force(e, g.ptr(dense), g.ptr(frc), 0, 0, 0, None, sp),
+                         "engine_force")
+            torch.cuda.synchronize()
+            assert g.rel_rms(frc.cpu().numpy().reshape(-1, 3), want) <= 1e-5
+            moved = dense.clone()
+            vel.zero_()
+            torch.cuda.synchronize()
+            torch.cuda._sleep(20_000_000)
+            g.capi.check(lib.snb_engine_set_prune_margin(e, ctypes.c_float(0.5)), "margin")
+            g.capi.check(lib.snb_engine_md_steps_graph(e, g.ptr(moved), g.ptr(vel), g.ptr(invm),
+                                                       dt, 1, 2, sp), "md")
+            torch.cuda.synchronize()
+            kick = dt.value * want
+            got = (vel.cpu().numpy() * packed.mass.repeat(3)).reshape(-1, 3)
+            assert g.rel_rms(got, 2 * kick) <= 0.05  # two short steps along the force
+    finally:
+        lib.snb_engine_destroy(e)
