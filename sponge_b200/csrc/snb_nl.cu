@@ -530,11 +530,8 @@ __device__ __forceinline__ float span_gap(int o, float lo, float hi) {
 // cells within reach of the group's box; 32 are tested at a time, one per
 // lane, against the group's atoms with the reference's criterion (the fast
 // |dr|^2 outside the band of k_pair_search, the exact one inside), and an
-// entry is kept when any pair passes.  The entry's mask leaves out exclusions
-// and, inside the group, the order j <= i; it does not record which pairs are
-// within r_l (nearly every mask is then full, which the pair kernel tests for
-// a whole batch; the pairs beyond r_l cannot come within the cutoff before
-// the next build), and the export tells them apart again.
+// entry is kept when any pair passes.  The entry's mask holds the pairs that
+// passed, without exclusions and, inside the group, the order j <= i.
 //
 // The entries of a row are stored nearest first: they are collected in shared
 // memory and counting-sorted by the smallest squared distance to the group
@@ -738,7 +735,7 @@ __global__ void __launch_bounds__(32 * kGroupSearchWarps) k_group_search(GroupSe
         // atoms of the group that j may pair with: all, or those before it
         unsigned may = 0xffu;
         if (j < g.x + g.y && j >= g.x) may = (1u << (j - g.x)) - 1u;
-        int hits = 0;
+        unsigned hits = 0u;
         float rmin = FLT_MAX;
         for (int ii = 0; ii < g.y; ++ii) {
           const float4 pi = sh_i[w][ii];
@@ -774,21 +771,18 @@ __global__ void __launch_bounds__(32 * kGroupSearchWarps) k_group_search(GroupSe
                 out = excluded_pair(min(gi, gj), max(gi, gj), a.excl_start, a.excl_list,
                                     a.excl_numbers);
             }
-            if (out) {
-              hit = false;
-              may &= ~(1u << ii);
-            }
+            hit = hit && !out;
           }
           if (hit) {
-            ++hits;
+            hits |= 1u << ii;
             rmin = fminf(rmin, r2);
           }
         }
-        pairs += hits;
-        const unsigned m = __ballot_sync(0xffffffffu, hits != 0);
-        if (hits != 0) {
+        pairs += __popc(hits);
+        const unsigned m = __ballot_sync(0xffffffffu, hits != 0u);
+        if (hits != 0u) {
           const int slot = held + __popc(m & lt);
-          se[slot] = ((unsigned)j << 8) | may;
+          se[slot] = ((unsigned)j << 8) | hits;
           sb[slot] = (unsigned char)min(31, (int)(rmin * bin_scale));
         }
         held += __popc(m);
@@ -1754,38 +1748,22 @@ int nl_export_atom_groups(NeighborList& nl, void* d_groups, int* d_slab,
   return kOk;
 }
 
-// Pairs of the grouped rows in global ids (lo, hi), in no particular order:
-// the entries' pairs that meet the criterion at the build-time coordinates.
+// Pairs of the grouped rows in global ids (lo, hi), in no particular order.
 __global__ void k_export_group_pairs(int ngroups, const int2* __restrict__ group,
                                      const int* __restrict__ row_count,
                                      const unsigned* __restrict__ entry, int cap_row,
-                                     const float4* __restrict__ pos, Cell cell, Cell rcell,
-                                     float rl2, BatchView bv, int* pi, int* pj, long long cap,
-                                     unsigned long long* next) {
+                                     const int* __restrict__ global, int* pi, int* pj,
+                                     long long cap, unsigned long long* next) {
   const int id = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (id >= ngroups || group[id].y == 0) return;
   const int2 g = group[id];
-  if (bv.nsys > 0) {
-    const SysGeom& s = bv.sys[bv.sys_of[g.x]];
-    cell = s.cell;
-    rcell = s.rcell;
-  }
   for (int k = lane; k < row_count[id]; k += 32) {
     const unsigned e = entry[(size_t)id * cap_row + k];
-    const float4 rj = pos[e >> 8];
-    const int gj = __float_as_int(rj.w);
+    const int gj = global[e >> 8];
     for (int b = 0; b < g.y; ++b) {
       if (!((e >> b) & 1u)) continue;
-      const float4 ri = pos[g.x + b];
-      const int gi = __float_as_int(ri.w);
-      float dx = __fsub_rn(ri.x, rj.x), dy = __fsub_rn(ri.y, rj.y), dz = __fsub_rn(ri.z, rj.z);
-      if (gj < gi) {
-        dx = -dx;
-        dy = -dy;
-        dz = -dz;
-      }
-      if (!(norm2_exact(min_image_exact_rect(dx, dy, dz, cell, rcell)) < rl2)) continue;
+      const int gi = global[g.x + b];
       const unsigned long long o = atomicAdd(next, 1ull);
       if ((long long)o < cap) {
         pi[o] = gi < gj ? gi : gj;
@@ -1837,8 +1815,8 @@ int nl_export_pairs(NeighborList& nl, int* d_pi, int* d_pj, long long cap,
     SNB_CUDA_TRY(cudaMalloc(&next, sizeof(unsigned long long)));
     SNB_CUDA_TRY(cudaMemsetAsync(next, 0, sizeof(unsigned long long), st));
     k_export_group_pairs<<<ceil_div(nl.max_groups, 8), 256, 0, st>>>(
-        nl.max_groups, nl.d_group, nl.d_grow_count, nl.d_gentry, nl.gcap, nl.d_pos, nl.cell,
-        nl.rcell, nl.rl2, nl.bv, d_pi, d_pj, cap, next);
+        nl.max_groups, nl.d_group, nl.d_grow_count, nl.d_gentry, nl.gcap, nl.d_global, d_pi,
+        d_pj, cap, next);
     cudaError_t e = cudaStreamSynchronize(st);
     cudaFree(next);
     if (e != cudaSuccess) return fail(kCudaError, cudaGetErrorString(e));

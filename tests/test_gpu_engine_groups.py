@@ -271,3 +271,31 @@ def test_regrown_rows_beside_default_stream_work(g, oracle):
             assert g.rel_rms(got, 2 * kick) <= 0.05  # two short steps along the force
     finally:
         lib.snb_engine_destroy(e)
+
+
+@pytest.mark.parametrize("waters,cutoff", [(900, 8.0), (300, 8.0)])
+def test_kept_list_holds_only_its_pairs(g, oracle, waters, cutoff):
+    """A list that is older than the displacement rule allows (rebuilt at an
+    interval instead): the forces are those of the pairs within cutoff + skin
+    at the build, whatever has come within the cutoff since beside them."""
+    from sponge_b200 import systems
+    s = systems.water_box(waters, seed=13)
+    rng = np.random.default_rng(13)
+    shift = np.repeat(rng.uniform(-0.25, 0.25, (s.n // 3 + 1, 3)), 3, axis=0)[:s.n]
+    moved = dataclasses.replace(s, crd=(s.crd + shift).astype(np.float32))
+    lib = g.capi.load()
+    e = g.engine_create(s, cutoff, skin=0.05, neighbor_list_refresh_interval=1000)
+    try:
+        _force_of(g, e, g.dev(s.crd.reshape(-1), np.float32), s.n, 0)
+        got = _force_of(g, e, g.dev(moved.crd.reshape(-1), np.float32), s.n, 1)
+    finally:
+        lib.snb_engine_destroy(e)
+    rs, cols = oracle.nl_pairs_system(s, cutoff, 0.05)
+    new_rs, new_cols = oracle.nl_pairs_system(moved, cutoff, 0.05)
+    beta = oracle.get_beta(cutoff)
+    other = (oracle.excluded_f64(moved, beta)["frc"] +
+             oracle.pme_f64(moved, (systems.fft_size(s.box),) * 3, beta)["frc"])
+    want = oracle.direct_f64(moved, cutoff, beta, rs, cols)["frc"] + other
+    fresh = oracle.direct_f64(moved, cutoff, beta, new_rs, new_cols)["frc"] + other
+    assert g.rel_rms(got, want) <= 1e-5
+    assert g.rel_rms(fresh, want) >= 5e-5  # the list's age shows at this tolerance
