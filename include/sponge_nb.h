@@ -495,7 +495,9 @@ int snb_engine_spread_wide_tiles(snb_engine* e, int* count, void* stream);
  * value is kept for snb_engine_list_form, 1 is refused where that form was
  * (a batch, a box below five cells per axis, the soft-core kernel), and the
  * next step rebuilds the list.  (Float accumulation, and boxes of 2^24 atoms
- * or more, keep a row of partners per atom, as snb_nl does.) */
+ * or more, keep a row of partners per atom, as snb_nl does; boxes whose rows
+ * per atom would exceed 32-bit offsets, 3.5 M atoms of water at cutoff 10 A and
+ * skin 2 A, are refused either way.) */
 int snb_engine_set_list_form(snb_engine* e, int clusters);
 /* Virtual atoms in the engine (NULL to remove): every force evaluation moves
  * the sites' forces onto their atoms before the forces are returned or the

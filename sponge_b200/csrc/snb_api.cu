@@ -2525,12 +2525,12 @@ extern "C" int snb_engine_spread_wide_tiles(snb_engine* e, int* count, void* str
 extern "C" int snb_engine_stats(snb_engine* e, long long* rebuilds, long long* pairs,
                                 void* stream) {
   if (!e) return fail(kBadInput, "engine_stats: null handle");
-  bool regrown;
-  int rc = nl_check_overflow(e->nl, &regrown, S(stream));
+  long long total = 0;
+  const int rc = nl_total_pairs(e->nl, &total, S(stream));
   engine_list_emptied(e);
   if (rc) return rc;
-  if (rebuilds) *rebuilds = e->nl.h_flags[3];
-  if (pairs) *pairs = e->nl.last_total;
+  if (rebuilds) *rebuilds = e->nl.h_flags[kFlagGeneration];
+  if (pairs) *pairs = total;
   return kOk;
 }
 

@@ -109,9 +109,10 @@ __device__ __forceinline__ bool box_rebuilds(const unsigned char* need, const in
   return need == nullptr || need[sys[i]] != 0;
 }
 
-// Device flags of a neighbor list (NeighborList::d_flags).  kFlagFull: the
-// pending rebuild covers every system of a batch (so the pair total restarts
-// from zero instead of being corrected row by row).
+// Device flags of a neighbor list (NeighborList::d_flags).  kFlagTotal: the
+// pairs of per-atom rows (32 bits hold them: the rows' offsets do).
+// kFlagFull: the pending rebuild covers every system of a batch (so that total
+// restarts from zero instead of being corrected row by row).
 enum { kFlagNeed = 0, kFlagListOverflow = 1, kFlagTotal = 2, kFlagGeneration = 3,
        kFlagExportOverflow = 4, kFlagMaxRow = 5, kFlagFull = 6, kNumFlags = 8 };
 
@@ -165,7 +166,8 @@ struct NeighborList {
   int* d_unsorted = nullptr;    // [n] cell-binned caller indices before ordering
   int* d_sorted_cell = nullptr;  // [n] cell of each sorted atom
   int* d_flags = nullptr;       // [0] need_update  [1] list overflow  [2] pair total
-                                // [3] rebuild count  [4] export overflow
+                                // [3] rebuild count  [4] export overflow; behind
+                                // the flags one 64-bit word for sums over groups
   int* h_flags = nullptr;       // pinned mirror
   ScanScratch scan;
   long long last_total = 0;

@@ -568,13 +568,7 @@ __global__ void __launch_bounds__(32 * kGroupSearchWarps) k_group_search(GroupSe
        id += gridDim.x * kGroupSearchWarps) {
     const int2 g = a.group[id];
     if (g.y == 0) {
-      if (lane == 0) a.row_count[id] = 0;
-      // a partial batch rebuild keeps the total of the other rows
-      if (lane == 0 && BATCH) {
-        if (a.flags[kFlagFull] == 0 && a.row_pairs[id] != 0)
-          atomicAdd(&a.flags[kFlagTotal], -a.row_pairs[id]);
-        a.row_pairs[id] = 0;
-      }
+      if (lane == 0) a.row_count[id] = a.row_pairs[id] = 0;
       continue;
     }
     if (BATCH && !box_rebuilds(a.bv.box_need, a.bv.sys_of, g.x)) continue;  // warp-uniform
@@ -796,11 +790,8 @@ __global__ void __launch_bounds__(32 * kGroupSearchWarps) k_group_search(GroupSe
     flush();
     pairs = __reduce_add_sync(0xffffffffu, pairs);
     if (lane == 0) {
-      // a partial batch rebuild replaces this row's share of the kept total
-      const int prev = (BATCH && a.flags[kFlagFull] == 0) ? a.row_pairs[id] : 0;
       a.row_count[id] = min(count, a.cap);
       a.row_pairs[id] = pairs;
-      atomicAdd(&a.flags[kFlagTotal], pairs - prev);
       if (count > a.cap) {
         a.flags[kFlagListOverflow] = 1;
         atomicMax(&a.flags[kFlagMaxRow], count);
@@ -1229,8 +1220,8 @@ static int nl_alloc(NeighborList& nl, int n, long long initial_capacity,
   SNB_CUDA_TRY(cudaMalloc(&nl.d_global, sizeof(int) * n));
   SNB_CUDA_TRY(cudaMalloc(&nl.d_pos, sizeof(float4) * n));
   SNB_CUDA_TRY(cudaMalloc(&nl.d_old_crd, sizeof(float3) * n));
-  SNB_CUDA_TRY(cudaMalloc(&nl.d_flags, sizeof(int) * kNumFlags));
-  SNB_CUDA_TRY(clear_now(nl.d_flags, sizeof(int) * kNumFlags));
+  SNB_CUDA_TRY(cudaMalloc(&nl.d_flags, sizeof(int) * (kNumFlags + 2)));
+  SNB_CUDA_TRY(clear_now(nl.d_flags, sizeof(int) * (kNumFlags + 2)));
   SNB_CUDA_TRY(cudaMallocHost(&nl.h_flags, sizeof(int) * kNumFlags));
   SNB_CUDA_TRY(cudaMalloc(&nl.d_unsorted, sizeof(int) * n));
   SNB_CUDA_TRY(cudaMalloc(&nl.d_sorted_cell, sizeof(int) * n));
@@ -1246,6 +1237,19 @@ static int nl_alloc(NeighborList& nl, int n, long long initial_capacity,
     SNB_CUDA_TRY(clear_now(nl.d_sorted_cell, sizeof(int) * n));
     SNB_CUDA_TRY(clear_now(nl.d_pos, sizeof(float4) * n));
   }
+  // Capacity of a row per atom: 1.5x (2.5x where cell pairs are owned by
+  // index, which balances rows less well) the mean half-sphere count plus a
+  // margin; regrown on overflow by nl_check_overflow.  Boxes whose rows exceed
+  // 32-bit offsets are refused in either form of the list (3.5 M atoms of
+  // water at cutoff 10 A, skin 2 A).
+  if (initial_capacity <= 0)
+    initial_capacity = (long long)((all_balanced ? 1.5 : 2.5) * max_per_atom) + 64;
+  nl.row_cap = (int)std::min<long long>(initial_capacity, n);
+  if (nl.row_cap < 32) nl.row_cap = 32;
+  nl.row_cap = (nl.row_cap + 7) & ~7;  // rows start on 32-byte boundaries
+  nl.cap = (long long)nl.row_cap * n;
+  if (nl.cap + nl.row_cap > 2147483647LL)
+    return fail(kBadInput, "neighbor list: rows exceed 32-bit offsets");
   if (groups && n < kGroupMaxAtoms) {
     nl.groups = true;
     // the row of a group of reach about 2 A: the half sphere of r_l + 2 A
@@ -1261,17 +1265,6 @@ static int nl_alloc(NeighborList& nl, int n, long long initial_capacity,
   SNB_CUDA_TRY(cudaMalloc(&nl.d_row_start, sizeof(int) * (n + 1)));
   SNB_CUDA_TRY(clear_now(nl.d_row_count, sizeof(int) * n));
   SNB_CUDA_TRY(clear_now(nl.d_row_start, sizeof(int) * (n + 1)));
-  // Row capacity: 1.5x (2.5x where cell pairs are owned by index, which
-  // balances rows less well) the mean half-sphere count plus a margin;
-  // regrown on overflow by nl_check_overflow.
-  if (initial_capacity <= 0)
-    initial_capacity = (long long)((all_balanced ? 1.5 : 2.5) * max_per_atom) + 64;
-  nl.row_cap = (int)std::min<long long>(initial_capacity, n);
-  if (nl.row_cap < 32) nl.row_cap = 32;
-  nl.row_cap = (nl.row_cap + 7) & ~7;  // rows start on 32-byte boundaries
-  nl.cap = (long long)nl.row_cap * n;
-  if (nl.cap + nl.row_cap > 2147483647LL)
-    return fail(kBadInput, "neighbor list: rows exceed 32-bit offsets");
   SNB_CUDA_TRY(cudaMalloc(&nl.d_cols, sizeof(int) * nl.cap));
   k_row_starts<<<ceil_div(n + 1, 256), 256>>>(n, nl.row_cap, nl.d_row_start);
   SNB_CUDA_TRY(cudaGetLastError());
@@ -1601,7 +1594,6 @@ int nl_check_overflow(NeighborList& nl, bool* regrown, cudaStream_t st) {
   SNB_CUDA_TRY(cudaMemcpyAsync(nl.h_flags, nl.d_flags, sizeof(int) * kNumFlags,
                                cudaMemcpyDeviceToHost, st));
   SNB_CUDA_TRY(cudaStreamSynchronize(st));
-  nl.last_total = nl.h_flags[kFlagTotal];
   if (!nl.h_flags[kFlagListOverflow]) return kOk;
   // The larger rows start out empty: whoever asked, the next update rebuilds
   // them (nl_decide forces what has no generation).
@@ -1633,11 +1625,54 @@ int nl_check_overflow(NeighborList& nl, bool* regrown, cudaStream_t st) {
   return kOk;
 }
 
-// The pairs of the last build (counted in full where the rows overflowed).
+// Sums over the groups: the pairs of their rows, or with mask the entries in
+// the batches of 32 that a prune pass kept.
+__global__ void k_sum_groups(int ngroups, const int2* __restrict__ group,
+                             const int* __restrict__ row_pairs,
+                             const int* __restrict__ row_count,
+                             const unsigned char* __restrict__ mask, int batches,
+                             unsigned long long* total) {
+  const int id = blockIdx.x * blockDim.x + threadIdx.x;
+  if (id >= ngroups || group[id].y == 0) return;
+  int n = 0;
+  if (mask) {
+    const int cnt = row_count[id];
+    for (int b = 0; 32 * b < cnt; ++b)
+      if (mask[(size_t)id * batches + b]) n += min(32, cnt - 32 * b);
+  } else {
+    n = row_pairs[id];
+  }
+  atomicAdd(total, (unsigned long long)n);
+}
+
+static int sum_groups(NeighborList& nl, const unsigned char* mask, long long* total,
+                      cudaStream_t st) {
+  auto* d = reinterpret_cast<unsigned long long*>(nl.d_flags + kNumFlags);
+  SNB_CUDA_TRY(cudaMemsetAsync(d, 0, sizeof(unsigned long long), st));
+  k_sum_groups<<<ceil_div(nl.max_groups, 256), 256, 0, st>>>(
+      nl.max_groups, nl.d_group, nl.d_gpairs, nl.d_grow_count, mask, nl.gcap / 32, d);
+  SNB_CUDA_TRY(cudaMemcpyAsync(total, d, sizeof(long long), cudaMemcpyDeviceToHost, st));
+  SNB_CUDA_TRY(cudaStreamSynchronize(st));
+  return kOk;
+}
+
+int nl_kept_entries(NeighborList& nl, long long* kept, cudaStream_t st) {
+  *kept = 0;
+  return nl.d_gmask ? sum_groups(nl, nl.d_gmask, kept, st) : kOk;
+}
+
+// The pairs of the last build (counted in full where the rows overflowed).  A
+// row's pairs fit 32 bits; their sum need not, so that of grouped rows is
+// formed here, before an overflow's regrowth empties them.
 int nl_total_pairs(NeighborList& nl, long long* total, cudaStream_t st) {
+  if (nl.groups && !nl.emptied) {
+    const int rc = sum_groups(nl, nullptr, &nl.last_total, st);
+    if (rc) return rc;
+  }
   bool regrown;
-  int rc = nl_check_overflow(nl, &regrown, st);
+  const int rc = nl_check_overflow(nl, &regrown, st);
   if (rc) return rc;
+  if (!nl.groups) nl.last_total = nl.h_flags[kFlagTotal];
   *total = nl.last_total;
   return kOk;
 }
@@ -1771,35 +1806,6 @@ __global__ void k_export_group_pairs(int ngroups, const int2* __restrict__ group
       }
     }
   }
-}
-
-// Entries in the batches of 32 that a prune pass kept.
-__global__ void k_kept_entries(int ngroups, const int2* __restrict__ group,
-                               const int* __restrict__ row_count,
-                               const unsigned char* __restrict__ mask, int batches,
-                               unsigned long long* total) {
-  const int id = blockIdx.x * blockDim.x + threadIdx.x;
-  if (id >= ngroups || group[id].y == 0) return;
-  int n = 0;
-  const int cnt = row_count[id];
-  for (int b = 0; 32 * b < cnt; ++b)
-    if (mask[(size_t)id * batches + b]) n += min(32, cnt - 32 * b);
-  atomicAdd(total, (unsigned long long)n);
-}
-
-int nl_kept_entries(NeighborList& nl, long long* kept, cudaStream_t st) {
-  *kept = 0;
-  if (!nl.d_gmask) return kOk;
-  unsigned long long* d = nullptr;
-  SNB_CUDA_TRY(cudaMalloc(&d, sizeof(unsigned long long)));
-  cudaMemsetAsync(d, 0, sizeof(unsigned long long), st);
-  k_kept_entries<<<ceil_div(nl.max_groups, 256), 256, 0, st>>>(
-      nl.max_groups, nl.d_group, nl.d_grow_count, nl.d_gmask, nl.gcap / 32, d);
-  cudaMemcpyAsync(kept, d, sizeof(long long), cudaMemcpyDeviceToHost, st);
-  const cudaError_t e = cudaStreamSynchronize(st);
-  cudaFree(d);
-  if (e != cudaSuccess) return fail(kCudaError, cudaGetErrorString(e));
-  return kOk;
 }
 
 int nl_export_pairs(NeighborList& nl, int* d_pi, int* d_pj, long long cap,

@@ -299,3 +299,25 @@ def test_kept_list_holds_only_its_pairs(g, oracle, waters, cutoff):
     fresh = oracle.direct_f64(moved, cutoff, beta, new_rs, new_cols)["frc"] + other
     assert g.rel_rms(got, want) <= 1e-5
     assert g.rel_rms(fresh, want) >= 5e-5  # the list's age shows at this tolerance
+
+
+def test_box_beyond_32_bit_rows_is_refused(g):
+    """1.2 M atoms at a cutoff of 20 A (2,230 pairs per atom): the list would
+    hold more than 2^31 pairs.  A row per atom never took such a box, and the
+    grouped rows do not either."""
+    lib = g.capi.load()
+    n, box = 1_200_000, (1_200_000 / 0.1) ** (1 / 3)
+    L = np.float32(box)
+    cell = np.array([L, 0, L, 0, 0, L], np.float32)
+    rcell = np.array([1 / L, 0, 1 / L, 0, 0, 1 / L], np.float32)
+    h = ctypes.c_void_p()
+    o = g.capi.options(cutoff=20.0, skin=2.0)
+    zero, none = np.zeros(n, np.int32), np.zeros(1, np.float32)
+    q = np.zeros(n, np.float32)
+    rc = lib.snb_engine_create(ctypes.byref(o), n, g.capi.boundary(cell, rcell), 1,
+                               zero.ctypes.data, none.ctypes.data, none.ctypes.data,
+                               q.ctypes.data, zero.ctypes.data, zero.ctypes.data,
+                               zero.ctypes.data, 0, ctypes.byref(h))
+    if rc == 0:
+        lib.snb_engine_destroy(h)
+    assert rc != 0 and b"32-bit offsets" in lib.snb_last_error()
