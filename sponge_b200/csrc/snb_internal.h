@@ -177,18 +177,20 @@ struct NeighborList {
   // atoms of one cell, whose atoms follow a path up and down the cell's four
   // xy quarter columns.  Row g lists the partner atoms with a pair within r_l
   // of group g as (sorted index << 8 | mask of the group's atoms), nearest
-  // first.  A cell's groups are numbered from cell_start / kGroupSize + cell,
-  // which leaves room for each cell's last, shorter group, so the numbers of
-  // a batch's systems do not depend on one another.  With groups the per-atom
-  // rows above are not allocated.
+  // first.  A cell's groups are numbered from cell_start / kGroupSize +
+  // min(cell, cell_start), which leaves room for each cell's last, shorter
+  // group, so the numbers of a batch's systems do not depend on one another,
+  // and a box of mostly empty cells has no more numbers than atoms.  With
+  // groups the per-atom rows above are not allocated.
   bool groups = false;
-  int max_groups = 0;
+  int max_groups = 0;            // numbers in use (some hold no atoms)
+  int group_room = 0;            // numbers the arrays hold (a redrawn grid keeps them)
   int* d_atom_key = nullptr;     // [n] caller frame: order key inside the cell
-  int2* d_group = nullptr;       // [max_groups] {first sorted atom, atom count}
-  int* d_grow_count = nullptr;   // [max_groups] entries of row g
-  int* d_gpairs = nullptr;       // [max_groups] pairs of row g
-  unsigned* d_gentry = nullptr;  // [max_groups * gcap]
-  unsigned char* d_gmask = nullptr;  // [max_groups * gcap / 32] (nl_enable_prune)
+  int2* d_group = nullptr;       // [group_room] {first sorted atom, atom count}
+  int* d_grow_count = nullptr;   // [group_room] entries of row g
+  int* d_gpairs = nullptr;       // [group_room] pairs of row g
+  unsigned* d_gentry = nullptr;  // [group_room * gcap]
+  unsigned char* d_gmask = nullptr;  // [group_room * gcap / 32] (nl_enable_prune)
   int gcap = 0;                  // a multiple of 32
 };
 constexpr int kGroupSize = 8;

@@ -167,6 +167,12 @@ __global__ void k_bin_scatter(int n, const int* __restrict__ atom_cell,
   }
 }
 
+// first_group(c, a): the number of cell c's first group, a atoms in the cells
+// before it.  A cell of m atoms gets at least ceil(m / 8) numbers: the first
+// term gives floor(m / 8), and the second rises by one wherever m > 0.  All
+// cells together take n / 8 + min(cells, n).
+__device__ __forceinline__ int first_group(int c, int a) { return a / kGroupSize + min(c, a); }
+
 // One warp per cell: order inside the cell by caller index (rank sort), or
 // by (key, caller index) when keys are given; with groups also the cell's
 // groups: as few as hold its atoms, of even sizes.
@@ -185,7 +191,7 @@ __global__ void k_cell_order(int ncell, const int* __restrict__ cell_start,
   if (group) {
     const int ng = (b - a + kGroupSize - 1) / kGroupSize;
     const int per = ng > 0 ? (b - a + ng - 1) / ng : 0;
-    const int id0 = a / kGroupSize + c, id1 = b / kGroupSize + c + 1;
+    const int id0 = first_group(c, a), id1 = first_group(c + 1, b);
     for (int t = lane; t < id1 - id0; t += 32)
       group[id0 + t] = make_int2(min(a + t * per, b - 1), max(0, min(per, b - a - t * per)));
   }
@@ -1176,14 +1182,18 @@ static void groups_free(NeighborList& nl) {
   nl.d_gmask = nullptr;
 }
 
+static int group_numbers(const NeighborList& nl) {  // see first_group
+  return nl.n / kGroupSize + std::min(nl.ncell, nl.n);
+}
+
 // Storage of the grouped rows for the current grid and row capacity gcap, with
 // every row empty for work that is queued on st afterwards.
 static int groups_alloc(NeighborList& nl, cudaStream_t st) {
   const bool pruned = nl.d_prune_ref != nullptr;
   groups_free(nl);
   nl.gcap = (std::max(nl.gcap, 32) + 31) & ~31;
-  nl.max_groups = nl.n / kGroupSize + nl.ncell;
-  const size_t G = nl.max_groups;
+  nl.max_groups = nl.group_room = group_numbers(nl);
+  const size_t G = nl.group_room;
   SNB_CUDA_TRY(cudaMalloc(&nl.d_atom_key, sizeof(int) * nl.n));
   SNB_CUDA_TRY(cudaMalloc(&nl.d_group, sizeof(int2) * G));
   SNB_CUDA_TRY(cudaMemsetAsync(nl.d_group, 0, sizeof(int2) * G, st));
@@ -1277,7 +1287,7 @@ static int nl_alloc(NeighborList& nl, int n, long long initial_capacity,
 int nl_enable_prune(NeighborList& nl, cudaStream_t st) {
   if (!nl.d_prune_ref) SNB_CUDA_TRY(cudaMalloc(&nl.d_prune_ref, sizeof(float4) * nl.n));
   if (nl.groups && !nl.d_gmask) {
-    const size_t bytes = (size_t)nl.max_groups * (nl.gcap / 32);
+    const size_t bytes = (size_t)nl.group_room * (nl.gcap / 32);
     SNB_CUDA_TRY(cudaMalloc(&nl.d_gmask, bytes));
     SNB_CUDA_TRY(cudaMemsetAsync(nl.d_gmask, 0, bytes, st));
   }
@@ -1377,7 +1387,8 @@ int nl_regrid(NeighborList& nl, const float* cell6) {
   nl.wy = c.a22 / nl.Ny;
   nl.iwz = nl.Nz / c.a33;
   nl.generation = 0;  // the next update rebuilds
-  if (nl.groups && nl.max_groups != nl.n / kGroupSize + nl.ncell) {
+  nl.max_groups = group_numbers(nl);
+  if (nl.groups && nl.max_groups > nl.group_room) {
     SNB_CUDA_TRY(cudaDeviceSynchronize());
     if ((rc = groups_alloc(nl, nullptr))) return rc;
     SNB_CUDA_TRY(cudaStreamSynchronize(nullptr));

@@ -321,3 +321,32 @@ def test_box_beyond_32_bit_rows_is_refused(g):
     if rc == 0:
         lib.snb_engine_destroy(h)
     assert rc != 0 and b"32-bit offsets" in lib.snb_last_error()
+
+
+def test_droplet_in_a_large_box_takes_rows_by_atoms(g, oracle):
+    """1,000 waters in a box of 85,000 cells: right, and held in rows for the
+    3,000 atoms (n / 8 + n rows of some 600 entries, 8 MB) instead of rows for
+    the cells (0.2 GB)."""
+    import torch
+    from sponge_b200 import systems
+    lib = g.capi.load()
+    s = dataclasses.replace(systems.water_box(1000, seed=3), box=200.0)
+    crd = g.dev(s.crd.reshape(-1), np.float32)
+
+    def run():
+        e = g.engine_create(s, 7.0, PM_grid_spacing=6.0)
+        _force_of(g, e, crd, s.n, 0)
+        return e
+
+    lib.snb_engine_destroy(run())  # modules loaded
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    e = run()
+    try:
+        used = free - torch.cuda.mem_get_info()[0]
+        got = _pairs(g, e)
+    finally:
+        lib.snb_engine_destroy(e)
+    rs, cols = oracle.nl_pairs_system(s, 7.0, 2.0)
+    assert np.array_equal(got, g.csr_to_pairs(rs, cols))
+    assert used < 100e6
