@@ -442,9 +442,7 @@ int snb_engine_profile_steps(snb_engine* e, float* crd, float* vel,
  * shape, times `steps` replays of the captured step graph (stream-launched
  * steps for the pair search's shape, or where the stream is the legacy
  * default one), each from the given coordinates, and keeps the fastest:
- * the pair kernel's persistent blocks per SM (occupancy maximum, 2, 3, in
- * blocks of 512 threads), the pair search's
- * blocks per SM (4, 8, 16), the PME gather's threads per block (128, 256,
+ * the pair search's blocks per SM (4, 8, 16), the PME gather's threads per block (128, 256,
  * 512), the PME spread's shape (tiles of edge 8 with 1, 2, 4 warps per
  * tile, or edge 0: int64 global atomics, no tiles; single box; edge 16 with
  * 4, 8 warps is only set by snb_engine_set_launch_shapes) and the PME
@@ -459,9 +457,10 @@ int snb_engine_profile_steps(snb_engine* e, float* crd, float* vel,
  * recaptures the step graph.  h_choice[0..8] receives {unroll, blocks per
  * SM (0 = occupancy maximum), search blocks per SM, gather threads, pair
  * warps per block, spread tile edge, spread warps per tile, hit stash (0 /
- * 1), own FFT (0 / 1)}; unroll, pair warps and the hit stash belong to
- * earlier pair kernels: they are kept as set and change nothing.  Allocates
- * scratch. */
+ * 1), own FFT (0 / 1)}.  Blocks per SM limits the pair kernel, in blocks of
+ * 512 threads (1 is below its occupancy, 0 and 2 or more are not); it is not
+ * tuned.  Unroll, pair warps and the hit stash belong to earlier pair kernels:
+ * they are kept as set and change nothing.  Allocates scratch. */
 int snb_engine_autotune(snb_engine* e, float* crd, float* vel,
                         const float* inverse_mass, float dt, int steps,
                         int* h_choice, void* stream);
@@ -491,10 +490,10 @@ int snb_engine_spread_wide_tiles(snb_engine* e, int* count, void* stream);
  * (neighbor_list.cpp:974-1025) as grouped rows: runs of up to eight atoms of
  * a cell, and per group the atoms with a pair within cutoff + skin, which the
  * pair kernel loads once for the whole group.  clusters = 0 / 1 chose between
- * two earlier forms of the list; both values now give the grouped rows.  The
- * value is kept for snb_engine_list_form, 1 is refused where that form was
- * (a batch, a box below five cells per axis, the soft-core kernel), and the
- * next step rebuilds the list.  (Float accumulation, and boxes of 2^24 atoms
+ * two earlier forms of the list; both values now give the grouped rows, and
+ * the call changes nothing.  The value is kept for snb_engine_list_form, and 1
+ * is refused where that form was (a batch, a box below five cells per axis, the
+ * soft-core kernel).  (Float accumulation, and boxes of 2^24 atoms
  * or more, keep a row of partners per atom, as snb_nl does; boxes whose rows
  * per atom would exceed 32-bit offsets, 3.5 M atoms of water at cutoff 10 A and
  * skin 2 A, are refused either way.) */

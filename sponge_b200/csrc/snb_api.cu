@@ -176,8 +176,9 @@ struct snb_engine {
   int* d_gtype = nullptr;
   SoftTables soft_tab;  // of `soft`; empty where its type tables are too large
   bool cluster_form = false;    // what snb_engine_list_form reports
-  // launch shapes: blocks per SM is tuned; the others are settings of pair
-  // kernels that are gone, kept for callers that set and read them back
+  // launch shapes of the pair kernel as callers set and read them back: blocks
+  // per SM limits it (launch_pair_groups), the others belonged to pair kernels
+  // that are gone
   int pair_unroll = 4;
   int pair_blocks_per_sm = 0;
   int pair_warps = 16;
@@ -2170,12 +2171,11 @@ extern "C" int snb_engine_profile_steps(snb_engine* e, float* crd, float* vel,
   return kOk;
 }
 
-// Times `steps` stream-launched steps from the same starting coordinates for
-// each candidate launch shape and keeps the fastest: the pair kernel's
-// persistent blocks per SM (occupancy maximum, 2, 3) by the whole
-// step (the PME branch shares the SMs with it), the pair
-// search's blocks per SM (4, 8, 16; a rebuild is forced every step), and the
-// gather's threads per block (128, 256, 512).  crd / vel are restored.
+// Times `steps` steps from the same starting coordinates for each candidate
+// launch shape and keeps the fastest: the pair search's blocks per SM (4, 8,
+// 16; a rebuild is forced every step), the gather's threads per block (128,
+// 256, 512), the spread's shape and the FFT by the whole step (the PME branch
+// shares the SMs with the pair kernel).  crd / vel are restored.
 extern "C" int snb_engine_autotune(snb_engine* e, float* crd, float* vel,
                                    const float* invm, float dt, int steps, int* h_choice,
                                    void* stream) {
@@ -2266,19 +2266,7 @@ extern "C" int snb_engine_autotune(snb_engine* e, float* crd, float* vel,
   };
   int rc = kOk;
   double best = 1e30, ms = 0.0;
-  // persistent blocks per SM of the pair kernel
-  int bb = 0;
-  for (int b : {0, 2, 3}) {
-    e->pair_blocks_per_sm = b;
-    if ((rc = measure_step(&ms))) break;
-    if (ms < best) {
-      best = ms;
-      bb = b;
-    }
-  }
-  e->pair_blocks_per_sm = bb;
   int bs = e->nl.search_blocks_per_sm;
-  best = 1e30;
   for (int b : {4, 8, 16}) {
     if (rc) break;
     e->nl.search_blocks_per_sm = b;
@@ -2460,8 +2448,6 @@ extern "C" int snb_engine_set_list_form(snb_engine* e, int clusters) {
                 "neighbor list: the cluster form needs one rectangular box of at least "
                 "five cells per axis");
   e->cluster_form = clusters != 0;
-  drop_graph(e);  // the captured step holds the previous list form
-  e->steps_done = 0;
   return kOk;
 }
 

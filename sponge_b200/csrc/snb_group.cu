@@ -164,8 +164,8 @@ __device__ __forceinline__ long long warp_sum_ll(long long x) {
   return x;
 }
 
-// Rows of the pair tables: 8 bytes an entry; flags of the row's atom.
-constexpr int kRowNoLJ = 1, kRowMarked = 2;
+// Rows of the pair tables: 8 bytes an entry; flag of the row's atom.
+constexpr int kRowNoLJ = 1;
 __device__ __forceinline__ float2 table_entry(const float2* t, int bytes) {
   return *reinterpret_cast<const float2*>(reinterpret_cast<const char*>(t) + (unsigned)bytes);
 }
@@ -241,8 +241,7 @@ k_lj_groups(GroupArgs a, Accumulators acc) {
       s[4] = -iz;
       s[6] = p.w;
       const bool lj = has_lj && lane < g.y;
-      reinterpret_cast<int*>(sh_t[w])[lane] =
-          ta + (lj ? 0 : kRowNoLJ) + (SOFT && tl < 0 ? kRowMarked : 0);
+      reinterpret_cast<int*>(sh_t[w])[lane] = ta + (lj ? 0 : kRowNoLJ);
       if (SOFT)
         reinterpret_cast<int*>(sh_tb[w])[lane] = ((tl >> 15) & 0x7fff) * a.n_types_b * 8;
     }
@@ -494,7 +493,8 @@ int launch_pair_groups(GroupArgs a, Accumulators& acc, bool energy, bool virial,
   int per_sm = 1;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32 * kGroupWarps, 0);
   per_sm = std::max(per_sm, 1);
-  // (the tuned counts of persistent blocks are in units of 512 threads)
+  // (a caller's limit is in units of 512 threads; five blocks of 128 fit, so
+  // only a limit of one is below the occupancy maximum)
   if (a.blocks_per_sm > 0) per_sm = std::min(per_sm, a.blocks_per_sm * (16 / kGroupWarps));
   // The rows of a small box are cut into parts until there are enough for the
   // 2,960 warps to have work (9,000 atoms: 26 us in two parts, 32 us whole);

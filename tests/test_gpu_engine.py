@@ -174,7 +174,7 @@ def test_autotune_keeps_results_bitwise(g, box_9k):
         st.synchronize()
         assert np.array_equal(crd.cpu().numpy(), c0)
         assert np.array_equal(vel.cpu().numpy(), v0)
-        assert choice[0] in (2, 4, 8) and choice[1] in (0, 2, 3)
+        assert choice[0] in (2, 4, 8) and choice[1] == 0  # not tuned: as set
         assert choice[2] in (4, 8, 16) and choice[3] in (128, 256, 512)
         assert choice[4] in (4, 8, 16)
         assert (choice[5], choice[6]) in ((8, 1), (8, 2), (8, 4), (0, 0))
@@ -305,6 +305,9 @@ def test_a_changed_engine_forgets_its_captured_step(g, small_box):
                                                          dt, 1 + 3 * k, 3, sp), "md")
             info = [ctypes.byref(x) for x in n]
             assert lib.snb_engine_graph_info(e, *info, sp) == 0 and n[0].value > 0
+            if k == 0:  # the list has one form: setting it keeps the step
+                assert lib.snb_engine_set_list_form(e, 0) == 0
+                assert lib.snb_engine_graph_info(e, *info, sp) == 0
             assert change() == 0
             assert lib.snb_engine_graph_info(e, *info, sp) != 0, k
         assert torch.isfinite(crd).all()
