@@ -145,7 +145,7 @@ struct NeighborList {
   int* d_excl_count = nullptr;
   int* d_excl_partner = nullptr;
   BatchView bv;                // nsys > 0: a batch of boxes (per-system grids)
-  int search_blocks_per_sm = 8;  // persistent blocks of the pair search per SM
+  int search_blocks_per_sm = 8;  // blocks of the pair search per SM (see nl_rebuild)
   // binning
   int* d_cell_count = nullptr;  // [ncell]
   int* d_cell_start = nullptr;  // [ncell + 1]

@@ -531,50 +531,72 @@ __device__ __forceinline__ float span_gap(int o, float lo, float hi) {
   return fmaxf(g, 0.f);
 }
 
-// One warp per group.  The candidates are the atoms of the own cell from the
+// W warps per group.  The candidates are the atoms of the own cell from the
 // group's first on and those of the runs the cell owns, each run cut to the
-// cells within reach of the group's box; 32 are tested at a time, one per
-// lane, against the group's atoms with the reference's criterion (the fast
-// |dr|^2 outside the band of k_pair_search, the exact one inside), and an
-// entry is kept when any pair passes.  The entry's mask holds the pairs that
-// passed, without exclusions and, inside the group, the order j <= i.
+// cells within reach of the group's box; they are dealt to the warps 32 at a
+// time and tested, one per lane, against the group's atoms with the reference's
+// criterion (the fast |dr|^2 outside the band of k_pair_search, the exact one
+// inside), and an entry is kept when any pair passes.  The entry's mask holds
+// the pairs that passed, without exclusions and, inside the group, the order
+// j <= i.
 //
 // The entries of a row are stored nearest first: they are collected in shared
 // memory and counting-sorted by the smallest squared distance to the group
-// (32 bins, in the order found within a bin), kGroupBuf at a time.  The pair
-// kernel then finds whole batches of 32 beyond the cutoff of two i atoms: on
-// liquid water at cutoff 10 A, skin 2 A, 80 of the 116 (batch, atom)
-// evaluations of a row remain, against 115 in the order of the cells (the
-// pair kernel: 161 us, against 167 us with 16 even bins and 173 us with 10).
+// (32 bins, in the order found within a bin), kGroupBuf at a time.  The row is
+// the same for every W.  The pair kernel then finds whole batches of 32 beyond
+// the cutoff of two i atoms: on liquid water at cutoff 10 A, skin 2 A, 80 of
+// the 116 (batch, atom) evaluations of a row remain, against 115 in the order
+// of the cells (the pair kernel: 161 us, against 167 us with 16 even bins and
+// 173 us with 10).
 //
-// One rebuild of the 99,639-atom box takes 0.45 ms where the search of a row
-// per atom took 0.49 ms; of a 648-atom box, whose 90 groups leave the chip
-// idle, it takes about 25 us more than that.  Loading the candidates a batch
-// ahead made no difference, one warp per block (fewer in flight) doubled it.
+// What bounds it is the chain of one group: its loads, its batches one after
+// another and the sort.  Launches in us (under ncu, cold) on 648, 1,299,
+// 3,000, 9,000 and 18,000 atoms: one warp per group 51, 83, 91, 73, 92; four
+// 21, 31, 35, 47, 78; eight 15, 22, 29, 53, 94; the search of a row per atom
+// 16, 26, 23, 41, 85.  Eight are taken while all groups are resident at once
+// (four blocks of eight warps per SM), four up to 48 groups per SM (a rebuild
+// of 36,000 atoms 154 us, with one warp 169-186), and one beyond (48,000 atoms
+// 219 us, with four 236).  More blocks than two rounds of the resident ones
+// would make the four warps faster still on the largest boxes (99,639 atoms:
+// 435 us with 64 per SM, 518 with 16, one warp 451), but they start on every
+// force call that keeps its list: 4-9 us there, 75 us on 1 M atoms.
 constexpr int kGroupBuf = 1024;
-constexpr int kGroupSearchWarps = 4;
+constexpr int kGroupSearchWarps = 4;  // warps per block
 
-template <bool BATCH>
-__global__ void __launch_bounds__(32 * kGroupSearchWarps) k_group_search(GroupSearchArgs a) {
+template <bool BATCH, int W>
+__global__ void __launch_bounds__(32 * (W > kGroupSearchWarps ? W : kGroupSearchWarps))
+    k_group_search(GroupSearchArgs a) {
   if (a.flags[kFlagNeed] == 0) return;
-  __shared__ float4 sh_i[kGroupSearchWarps][kGroupSize];  // relative to the first; global id
-  __shared__ float3 sh_raw[kGroupSearchWarps][kGroupSize];
-  __shared__ int4 sh_ex[kGroupSearchWarps][kGroupSize];   // partners: count, first two, lists
-  __shared__ unsigned sh_e[kGroupSearchWarps][kGroupBuf];
-  __shared__ unsigned char sh_b[kGroupSearchWarps][kGroupBuf];
-  __shared__ int sh_h[kGroupSearchWarps][32];
+  constexpr int kAtOnce = W > kGroupSearchWarps ? 1 : kGroupSearchWarps / W;
+  constexpr int kHold = kGroupBuf + 32 * (W - 1);
+  __shared__ float4 sh_i[kAtOnce][kGroupSize];  // relative to the first; global id
+  __shared__ float3 sh_raw[kAtOnce][kGroupSize];
+  __shared__ int4 sh_ex[kAtOnce][kGroupSize];   // partners: count, first two, lists
+  __shared__ unsigned sh_e[kAtOnce][kHold];
+  __shared__ unsigned char sh_b[kAtOnce][kHold];
+  __shared__ int sh_h[kAtOnce][W][32];
+  __shared__ int sh_n[W > 1 ? 2 : 1][W];        // hits of a round's batches, by turns
+  __shared__ int sh_p[W];
   const int lane = threadIdx.x & 31;
-  const int w = threadIdx.x >> 5;
+  const int w = (threadIdx.x >> 5) / W;         // group of the block
+  const int part = (threadIdx.x >> 5) % W;      // warp of the group
   const unsigned lt = (1u << lane) - 1u;
   unsigned* se = sh_e[w];
   unsigned char* sb = sh_b[w];
-  int* hist = sh_h[w];
+  int* hist = sh_h[w][part];
   const float bin_scale = 32.0f / a.rl2;
-  for (int id = blockIdx.x * kGroupSearchWarps + w; id < a.ngroups;
-       id += gridDim.x * kGroupSearchWarps) {
+  // a group's warps (W > 1: the whole block, which every branch around a sync
+  // takes as one)
+  auto sync = [] {
+    if (W == 1)
+      __syncwarp();
+    else
+      __syncthreads();
+  };
+  for (int id = blockIdx.x * kAtOnce + w; id < a.ngroups; id += gridDim.x * kAtOnce) {
     const int2 g = a.group[id];
     if (g.y == 0) {
-      if (lane == 0) a.row_count[id] = a.row_pairs[id] = 0;
+      if (lane == 0 && part == 0) a.row_count[id] = a.row_pairs[id] = 0;
       continue;
     }
     if (BATCH && !box_rebuilds(a.bv.box_need, a.bv.sys_of, g.x)) continue;  // warp-uniform
@@ -612,8 +634,8 @@ __global__ void __launch_bounds__(32 * kGroupSearchWarps) k_group_search(GroupSe
                        m > 1 ? a.excl_partner[gl * kExclCap + 1] : -1, 0);
       }
     }
-    __syncwarp();
-    if (lane < kGroupSize) {
+    sync();
+    if (lane < kGroupSize && part == 0) {
       sh_i[w][lane] = make_float4(ix, iy, iz, p.w);
       sh_raw[w][lane] = make_float3(p.x, p.y, p.z);
       sh_ex[w][lane] = ex;
@@ -642,39 +664,47 @@ __global__ void __launch_bounds__(32 * kGroupSearchWarps) k_group_search(GroupSe
       hz = fmaxf(hz, __shfl_xor_sync(0xffffffffu, hz, o));
     }
     const bool wide = !(slack > a.rl * 1.0001f);
-    __syncwarp();
-    int count = 0, held = 0, pairs = 0;
+    sync();
+    int count = 0, held = 0, pairs = 0, round = 0;
     unsigned* out = a.entry + (size_t)id * a.cap;
-    // counting sort of the held entries onto the row's end
-    auto flush = [&]() {
+    // counting sort of the first m held entries onto the row's end, each warp a
+    // stretch of them
+    auto flush = [&](int m) {
+      const int stretch = W == 1 ? m : (m + 32 * W - 1) / (32 * W) * 32;
+      const int k1 = min(m, (part + 1) * stretch);
       hist[lane] = 0;
       __syncwarp();
-      for (int k = lane; k < held; k += 32) atomicAdd(&hist[sb[k]], 1);
-      __syncwarp();
-      const int own = hist[lane];
+      for (int k = part * stretch + lane; k < k1; k += 32) atomicAdd(&hist[sb[k]], 1);
+      sync();
+      // the bin's entries in all stretches, and in those before this one
+      int own = 0, earlier = 0;
+#pragma unroll
+      for (int k = 0; k < W; ++k) {
+        const int v = sh_h[w][k][lane];
+        own += v;
+        if (k < part) earlier += v;
+      }
       int incl = own;
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
         const int v = __shfl_up_sync(0xffffffffu, incl, o);
         if (lane >= o) incl += v;
       }
+      sync();
+      hist[lane] = incl - own + earlier;
       __syncwarp();
-      hist[lane] = incl - own;
-      __syncwarp();
-      for (int k0 = 0; k0 < held; k0 += 32) {
+      for (int k0 = part * stretch; k0 < k1; k0 += 32) {
         const int k = k0 + lane;
-        const int b = k < held ? sb[k] : 32;
+        const int b = k < k1 ? sb[k] : 32;
         const unsigned peers = __match_any_sync(0xffffffffu, b);
-        if (k < held) {
+        if (k < k1) {
           const int slot = count + hist[b] + __popc(peers & lt);
           if (slot < a.cap) out[slot] = se[k];
         }
         __syncwarp();
-        if (k < held && (peers & lt) == 0) hist[b] += __popc(peers);
+        if (k < k1 && (peers & lt) == 0) hist[b] += __popc(peers);
         __syncwarp();
       }
-      count += held;
-      held = 0;
     };
     const int nr = a.run_count[c];
     for (int r0 = -1; r0 < nr; r0 += 32) {
@@ -715,7 +745,8 @@ __global__ void __launch_bounds__(32 * kGroupSearchWarps) k_group_search(GroupSe
       const int excl = incl - len;
       const int nq = min(32, nr - r0);
       int cursor = 0;
-      for (int base = 0; base < total; base += 32) {
+      for (int base0 = 0; base0 < total; base0 += 32 * W) {
+        const int base = base0 + 32 * part;
         const int fi = base + lane;
         int j = -1;
         for (int q = cursor; q < nq; ++q) {  // warp-uniform
@@ -737,7 +768,7 @@ __global__ void __launch_bounds__(32 * kGroupSearchWarps) k_group_search(GroupSe
         if (j < g.x + g.y && j >= g.x) may = (1u << (j - g.x)) - 1u;
         unsigned hits = 0u;
         float rmin = FLT_MAX;
-        for (int ii = 0; ii < g.y; ++ii) {
+        for (int ii = 0; ii < g.y && base < total; ++ii) {
           const float4 pi = sh_i[w][ii];
           float dx = jx - pi.x, dy = jy - pi.y, dz = jz - pi.z;
           if (wide) {
@@ -780,22 +811,60 @@ __global__ void __launch_bounds__(32 * kGroupSearchWarps) k_group_search(GroupSe
         }
         pairs += __popc(hits);
         const unsigned m = __ballot_sync(0xffffffffu, hits != 0u);
+        // the round's batches follow one another; the buffer is emptied after
+        // the batch that fills it, as one warp alone would do it
+        int before = held, after = held, full = 0;
+        if (W == 1) {
+          after += __popc(m);
+          full = after > kGroupBuf - 32 ? after : 0;
+        } else {
+          int* n = sh_n[round & (W > 1 ? 1 : 0)];
+          ++round;
+          if (lane == 0) n[part] = __popc(m);
+          __syncthreads();
+#pragma unroll
+          for (int k = 0; k < W; ++k) {
+            if (k < part) before += n[k];
+            after += n[k];
+            if (full == 0 && after > kGroupBuf - 32) full = after;
+          }
+        }
         if (hits != 0u) {
-          const int slot = held + __popc(m & lt);
+          const int slot = before + __popc(m & lt);
           se[slot] = ((unsigned)j << 8) | hits;
           sb[slot] = (unsigned char)min(31, (int)(rmin * bin_scale));
         }
-        held += __popc(m);
-        if (held > kGroupBuf - 32) {
-          __syncwarp();
-          flush();
+        held = after;
+        if (full != 0) {
+          sync();
+          flush(full);
+          count += full;
+          held -= full;
+          if (W > 1) {  // the entries of the batches behind it move to the front
+            __syncthreads();
+            const int k = threadIdx.x;
+            const unsigned e = k < held ? se[full + k] : 0u;
+            const unsigned char b = k < held ? sb[full + k] : 0;
+            __syncthreads();
+            if (k < held) {
+              se[k] = e;
+              sb[k] = b;
+            }
+          }
         }
       }
     }
-    __syncwarp();
-    flush();
     pairs = __reduce_add_sync(0xffffffffu, pairs);
-    if (lane == 0) {
+    if (W > 1 && lane == 0) sh_p[part] = pairs;
+    sync();
+    flush(held);
+    count += held;
+    if (lane == 0 && part == 0) {
+      if (W > 1) {
+        pairs = 0;
+#pragma unroll
+        for (int k = 0; k < W; ++k) pairs += sh_p[k];
+      }
       a.row_count[id] = min(count, a.cap);
       a.row_pairs[id] = pairs;
       if (count > a.cap) {
@@ -1543,12 +1612,18 @@ int nl_rebuild(NeighborList& nl, const float* crd_f, const int* atom_local,
     ga.entry = nl.d_gentry;
     ga.flags = nl.d_flags;
     ga.bv = nl.bv;
-    const int gblocks = std::min(ceil_div(nl.max_groups, kGroupSearchWarps),
-                                 sms * std::max(1, nl.search_blocks_per_sm));
-    if (nl.bv.nsys > 0)
-      k_group_search<true><<<gblocks, 32 * kGroupSearchWarps, 0, st>>>(ga);
-    else
-      k_group_search<false><<<gblocks, 32 * kGroupSearchWarps, 0, st>>>(ga);
+    // (the warps per group: see k_group_search)
+    const int per_sm = std::max(1, nl.search_blocks_per_sm);
+    const int W = nl.max_groups <= 4 * sms ? 8 : (nl.max_groups <= 48 * sms ? 4 : 1);
+    auto search = nl.bv.nsys > 0 ? (W == 8   ? k_group_search<true, 8>
+                                    : W == 4 ? k_group_search<true, 4>
+                                             : k_group_search<true, 1>)
+                                 : (W == 8   ? k_group_search<false, 8>
+                                    : W == 4 ? k_group_search<false, 4>
+                                             : k_group_search<false, 1>);
+    const int gblocks = W == 1 ? std::min(ceil_div(nl.max_groups, kGroupSearchWarps), sms * per_sm)
+                               : std::min(nl.max_groups, sms * 2 * per_sm);
+    search<<<gblocks, 32 * std::max(W, kGroupSearchWarps), 0, st>>>(ga);
     k_finish_build<<<1, 1, 0, st>>>(nl.d_flags);
     if (need)  // the systems' flags for the next decision
       SNB_CUDA_TRY(cudaMemsetAsync(nl.bv.box_need, 0, nl.bv.nsys, st));

@@ -104,11 +104,26 @@ def _check(g, oracle, s, cutoff, tol=1e-5):
     (700, 7.3, 1e-5),    # 5 cells per axis: trimmed runs, some groups imaged
     (1500, 9.0, 1e-9),   # beta * cutoff = 4.3: beyond the polynomial
     (2600, 6.1, 1e-5),   # narrow cells: groups of a few atoms
+    (1400, 15.0, 1e-5),  # rows beyond the search's buffer, eight warps per group
+    (1700, 15.0, 1e-5),  # the same with four
 ])
 def test_groups_match_fp64(g, oracle, waters, cutoff, tol):
     from sponge_b200 import systems
     s = systems.water_box(waters, seed=waters, ion_pairs=None)
     _check(g, oracle, s, cutoff, tol)
+
+
+def test_long_rows_of_a_large_box(g, oracle):
+    """Rows beyond the search's buffer where one warp takes a group."""
+    from sponge_b200 import systems
+    s = systems.water_box(19500, seed=4, ion_pairs=None)
+    lib = g.capi.load()
+    e = g.engine_create(s, 15.0)
+    try:
+        got = _force_of(g, e, g.dev(s.crd.reshape(-1), np.float32), s.n, 0)
+    finally:
+        lib.snb_engine_destroy(e)
+    assert g.rel_rms(got, _want(oracle, s, 15.0)) <= 1e-5
 
 
 def test_sparse_and_dense_cells(g, oracle):
