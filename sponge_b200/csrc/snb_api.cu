@@ -1461,7 +1461,7 @@ static int engine_forces(snb_engine* e, const float* crd, int step, bool energy,
   const bool do_pme = e->pme.reciprocal && step % e->pme.update_interval == 0;
   const bool groups = e->nl.groups;
   const int* types = !groups ? e->lj.d_type : (e->soft ? e->soft_tab.type : e->d_gtype);
-  if (e->soft && (!groups || !types))
+  if (e->soft && (!groups || !types || !e->nl.mark_type))
     return fail(kNotSupported, "soft-core rows: type tables too large");
   if (do_pme)
     rc = pme_pack_bin(e->pme, e->n, reinterpret_cast<const float3*>(crd), e->d_charge, types,
@@ -1471,34 +1471,9 @@ static int engine_forces(snb_engine* e, const float* crd, int step, bool energy,
                      e->nl.d_perm, e->d_pos, e->d_type_sorted, st);
   if (rc) return rc;
   prof_mark(e, 2, st);
-  const bool fork = !e->prof_on;
-  cudaStream_t sb = fork ? e->branch : st;
-  if (fork) {
-    // PME on `branch`, the excluded correction and bonded terms on `branch2`,
-    // the pair kernel on the step's stream
-    cudaStream_t sb2 = e->branch2;
-    SNB_CUDA_TRY(cudaEventRecord(e->ev_fork, st));
-    SNB_CUDA_TRY(cudaStreamWaitEvent(sb, e->ev_fork, 0));
-    SNB_CUDA_TRY(cudaStreamWaitEvent(sb2, e->ev_fork, 0));
-    if (with_bonded && (rc = engine_bonded(e, crd, sb2))) return rc;
-    if (e->pme.excluded &&
-        (rc = launch_excluded(e->n, reinterpret_cast<const float3*>(crd), e->d_charge,
-                              e->cell, e->rcell, e->pme.beta, e->d_excl_start,
-                              e->d_excl_list, e->d_excl_numbers, e->nl.d_inv_perm, e->acc,
-                              e->accum, energy, virial, sb2, e->bv)))
-      return rc;
-    if (e->nb14 &&
-        (rc = launch_nb14(e->nb14->p, reinterpret_cast<const float3*>(crd), e->d_charge,
-                          e->cell, e->rcell, e->nl.d_inv_perm, e->acc, energy, virial, false,
-                          energy ? e->d_nb14_sums : nullptr, sb2)))
-      return rc;
-    SNB_CUDA_TRY(cudaEventRecord(e->ev_join2, sb2));
-    if (do_pme && (rc = pme_after_bin(e->pme, e->n, e->acc, e->accum, energy, virial, sb)))
-      return rc;
-    SNB_CUDA_TRY(cudaEventRecord(e->ev_join, sb));
-  }
+  GroupArgs ga;
   if (groups) {
-    GroupArgs a;
+    GroupArgs& a = ga;
     a.n = e->n;
     a.ngroups = e->nl.max_groups;
     a.group = e->nl.d_group;
@@ -1522,6 +1497,8 @@ static int engine_forces(snb_engine* e, const float* crd, int step, bool energy,
       a.n_types = e->soft->nA;
       a.lj_b = e->soft_tab.b;
       a.n_types_b = e->soft->nB;
+      a.marked = e->nl.d_marked;
+      a.nmarked = e->nl.d_nmarked;
       a.lambda = e->soft->lambda;
       a.alp_A = e->soft->alpha * powf(e->soft->lambda, e->soft->p);
       a.alp_B = e->soft->alpha * powf(1.0f - e->soft->lambda, e->soft->p);
@@ -1541,7 +1518,38 @@ static int engine_forces(snb_engine* e, const float* crd, int step, bool energy,
     } else if ((rc = engine_prune_invalidate(e, st))) {
       return rc;
     }
-    rc = launch_pair_groups(a, e->acc, energy, virial, st);
+  }
+  const bool fork = !e->prof_on;
+  cudaStream_t sb = fork ? e->branch : st;
+  if (fork) {
+    // PME on `branch`, the excluded correction and bonded terms on `branch2`,
+    // the pair kernel on the step's stream
+    cudaStream_t sb2 = e->branch2;
+    SNB_CUDA_TRY(cudaEventRecord(e->ev_fork, st));
+    SNB_CUDA_TRY(cudaStreamWaitEvent(sb, e->ev_fork, 0));
+    SNB_CUDA_TRY(cudaStreamWaitEvent(sb2, e->ev_fork, 0));
+    if (e->soft && (rc = launch_marked_groups(ga, e->acc, energy, virial, sb2))) return rc;
+    if (with_bonded && (rc = engine_bonded(e, crd, sb2))) return rc;
+    if (e->pme.excluded &&
+        (rc = launch_excluded(e->n, reinterpret_cast<const float3*>(crd), e->d_charge,
+                              e->cell, e->rcell, e->pme.beta, e->d_excl_start,
+                              e->d_excl_list, e->d_excl_numbers, e->nl.d_inv_perm, e->acc,
+                              e->accum, energy, virial, sb2, e->bv)))
+      return rc;
+    if (e->nb14 &&
+        (rc = launch_nb14(e->nb14->p, reinterpret_cast<const float3*>(crd), e->d_charge,
+                          e->cell, e->rcell, e->nl.d_inv_perm, e->acc, energy, virial, false,
+                          energy ? e->d_nb14_sums : nullptr, sb2)))
+      return rc;
+    SNB_CUDA_TRY(cudaEventRecord(e->ev_join2, sb2));
+    if (do_pme && (rc = pme_after_bin(e->pme, e->n, e->acc, e->accum, energy, virial, sb)))
+      return rc;
+    SNB_CUDA_TRY(cudaEventRecord(e->ev_join, sb));
+  }
+  if (groups) {
+    if (e->soft && !fork && (rc = launch_marked_groups(ga, e->acc, energy, virial, st)))
+      return rc;
+    rc = launch_pair_groups(ga, e->acc, energy, virial, st);
   } else {
     PairArgs a;
     a.n = e->n;
@@ -1870,11 +1878,17 @@ extern "C" int snb_engine_set_soft_core(snb_engine* e, snb_lj_soft* soft) {
     // a failure here leaves the engine with the module it had
     SNB_CUDA_TRY(cudaDeviceSynchronize());  // steps queued with the previous tables
     SoftTables t;
-    const int rc = engine_soft_tables(soft, &t);
+    int rc = engine_soft_tables(soft, &t);
+    if (!rc && (rc = nl_set_marks(e->nl, t.type))) {
+      nl_set_marks(e->nl, e->soft ? e->soft_tab.type : nullptr);
+      t.release();
+    }
     if (rc) return rc;
     e->soft_tab.release();
     e->soft_tab = t;
     e->cluster_form = false;
+  } else if (e->soft) {
+    nl_set_marks(e->nl, nullptr);
   }
   e->soft = soft;
   if (soft) {

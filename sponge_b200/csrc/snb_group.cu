@@ -179,7 +179,17 @@ __device__ __forceinline__ float2 image2(float2 d, float L, float rL) {
   return make_float2(min_image_axis(d.x, L, rL), min_image_axis(d.y, L, rL));
 }
 
-template <bool ENERGY, bool VIRIAL, bool BATCH, bool SOFT, bool FAR>
+// SOFT: plain LJ, or of a soft-core box the rows of groups without a marked
+// atom, or those with one.  Nearly all pairs of a marked row take the soft-core
+// terms, so one such row by one warp outlasts the rest of the launch on boxes
+// of less than 50,000 atoms: the marked rows have a launch of their own beside
+// the others, in parts of about a batch (step of 7,500, 19,200, 38,000 and
+// 300,000 atoms with 35 to 64 marked sites: 56, 100, 114 and 594 us, in one
+// launch with whole rows 78, 112, 137 and 599; marked rows in parts at the
+// start of one launch, with more registers spilled: -, 98, 116 and 620).
+enum { kNoSoft, kPlainRows, kMarkedRows };
+
+template <bool ENERGY, bool VIRIAL, bool BATCH, int SOFT, bool FAR>
 __global__ void __launch_bounds__(32 * kGroupWarps, ENERGY || VIRIAL ? 1 : 5)
 k_lj_groups(GroupArgs a, Accumulators acc) {
   // a group's atoms by pairs: {-x0, -x1, -y0, -y1}, {-z0, -z1, q0, q1}
@@ -209,14 +219,22 @@ k_lj_groups(GroupArgs a, Accumulators acc) {
     src[r] = (lane + 32 * r) / 3;
     axis[r] = ((lane + 32 * r) - 3 * src[r]) * acc.fc;
   }
-  const int units = a.ngroups << a.split_log2;
+  // the marked rows are cut into parts of about a batch
+  int units = a.ngroups << a.split_log2, split = a.split_log2;
+  if (SOFT == kMarkedRows) {
+    const int m = *a.nmarked;
+    for (split = 4; split > 0 && (m << split) > (int)gridDim.x * kGroupWarps; --split) {
+    }
+    units = m << split;
+  }
   for (int u = blockIdx.x * kGroupWarps + w; u < units; u += gridDim.x * kGroupWarps) {
-    const int id = u >> a.split_log2, part = u & ((1 << a.split_log2) - 1);
+    const int part = u & ((1 << split) - 1);
+    const int id = SOFT == kMarkedRows ? a.marked[u >> split] : u >> split;
     const int2 g = a.group[id];
     if (g.y == 0) continue;
     const int cnt = a.row_count[id];
     const int nb = (cnt + 31) >> 5;
-    const int b0 = (nb * part) >> a.split_log2, b1 = (nb * (part + 1)) >> a.split_log2;
+    const int b0 = (nb * part) >> split, b1 = (nb * (part + 1)) >> split;
     if (b0 == b1 && !(pass && part == 0)) continue;
     const SysGeom* gs = BATCH ? a.bv.sys + a.bv.sys_of[g.x] : nullptr;
     const float Lx = BATCH ? gs->cell.a11 : a.cell.a11, rLx = BATCH ? gs->rcell.a11 : a.rcell.a11;
@@ -230,6 +248,7 @@ k_lj_groups(GroupArgs a, Accumulators acc) {
                 cz = __shfl_sync(0xffffffffu, p.z, 0);
     const float ix = min_image_axis(p.x - cx, Lx, rLx), iy = min_image_axis(p.y - cy, Ly, rLy),
                 iz = min_image_axis(p.z - cz, Lz, rLz);
+    if (SOFT == kPlainRows && __any_sync(0xffffffffu, tl < 0)) continue;
     const int ta = (SOFT ? tl & 0x7fff : tl & ~kTypeNoLJ) * a.n_types * 8;
     const bool has_lj = !(tl & kTypeNoLJ);
     __syncwarp();
@@ -245,7 +264,6 @@ k_lj_groups(GroupArgs a, Accumulators acc) {
       if (SOFT)
         reinterpret_cast<int*>(sh_tb[w])[lane] = ((tl >> 15) & 0x7fff) * a.n_types_b * 8;
     }
-    const bool mixed = SOFT && __any_sync(0xffffffffu, tl < 0);
     // The partners are taken in the image nearest to the first atom.  That
     // image is the nearest one to every i atom too, for all pairs within
     // rmax, when rmax plus the group's reach along an axis stays below half
@@ -254,7 +272,7 @@ k_lj_groups(GroupArgs a, Accumulators acc) {
 #pragma unroll
     for (int o = 4; o > 0; o >>= 1) slack = fminf(slack, __shfl_xor_sync(0xffffffffu, slack, o));
     const bool wide = !(slack > rmax * 1.0001f);
-    const bool general = wide || mixed;
+    const bool general = wide || SOFT == kMarkedRows;
     __syncwarp();
     float2 f[4][3];
 #pragma unroll
@@ -467,7 +485,7 @@ k_lj_groups(GroupArgs a, Accumulators acc) {
 
 using GroupKern = void (*)(GroupArgs, Accumulators);
 
-template <bool BATCH, bool SOFT, bool FAR>
+template <bool BATCH, int SOFT, bool FAR>
 static GroupKern group_kernel(bool energy, bool virial) {
   return energy ? (virial ? k_lj_groups<true, true, BATCH, SOFT, FAR>
                           : k_lj_groups<true, false, BATCH, SOFT, FAR>)
@@ -476,20 +494,40 @@ static GroupKern group_kernel(bool energy, bool virial) {
 }
 
 template <bool FAR>
-static GroupKern group_kernel(bool batch, bool soft, bool energy, bool virial) {
-  return soft    ? group_kernel<false, true, FAR>(energy, virial)
-         : batch ? group_kernel<true, false, FAR>(energy, virial)
-                 : group_kernel<false, false, FAR>(energy, virial);
+static GroupKern group_kernel(bool batch, int soft, bool energy, bool virial) {
+  return soft == kPlainRows    ? group_kernel<false, kPlainRows, FAR>(energy, virial)
+         : soft == kMarkedRows ? group_kernel<false, kMarkedRows, FAR>(energy, virial)
+         : batch               ? group_kernel<true, kNoSoft, FAR>(energy, virial)
+                               : group_kernel<false, kNoSoft, FAR>(energy, virial);
+}
+
+static GroupKern group_kernel(const GroupArgs& a, int soft, bool energy, bool virial) {
+  const bool batch = a.bv.nsys > 0;
+  return a.beta * a.cutoff > 4.0f ? group_kernel<true>(batch, soft, energy, virial)
+                                  : group_kernel<false>(batch, soft, energy, virial);
+}
+
+static int multiprocessors() {
+  static int sms = 0;
+  if (!sms) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, 0);
+  return sms;
+}
+
+int launch_marked_groups(GroupArgs a, Accumulators& acc, bool energy, bool virial,
+                         cudaStream_t st) {
+  if (a.n <= 0) return kOk;
+  const int blocks = std::min(ceil_div((long long)a.ngroups << 4, kGroupWarps),
+                              multiprocessors());
+  group_kernel(a, kMarkedRows, energy, virial)<<<blocks, 32 * kGroupWarps, 0, st>>>(a, acc);
+  SNB_CUDA_TRY(cudaGetLastError());
+  return kOk;
 }
 
 int launch_pair_groups(GroupArgs a, Accumulators& acc, bool energy, bool virial,
                        cudaStream_t st) {
   if (a.n <= 0) return kOk;
-  const bool soft = a.lj_b != nullptr, batch = a.bv.nsys > 0;
-  GroupKern kern = a.beta * a.cutoff > 4.0f ? group_kernel<true>(batch, soft, energy, virial)
-                                            : group_kernel<false>(batch, soft, energy, virial);
-  static int sms = 0;
-  if (!sms) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, 0);
+  GroupKern kern = group_kernel(a, a.lj_b ? kPlainRows : kNoSoft, energy, virial);
+  const int sms = multiprocessors();
   int per_sm = 1;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32 * kGroupWarps, 0);
   per_sm = std::max(per_sm, 1);

@@ -192,6 +192,10 @@ struct NeighborList {
   unsigned* d_gentry = nullptr;  // [group_room * gcap]
   unsigned char* d_gmask = nullptr;  // [group_room * gcap / 32] (nl_enable_prune)
   int gcap = 0;                  // a multiple of 32
+  // groups with a marked atom (nl_set_marks), listed at each build
+  const int* mark_type = nullptr;  // [n] caller frame, negative: marked; or null
+  int* d_marked = nullptr;       // [group_room]
+  int* d_nmarked = nullptr;      // [1]
 };
 constexpr int kGroupSize = 8;
 constexpr int kGroupMaxAtoms = 1 << 24;  // sorted indices that an entry holds
@@ -209,6 +213,9 @@ void nl_free(NeighborList& nl);
 // Allocates what the pruned rows need (the kept-atom bytes of grouped rows,
 // cleared on st).
 int nl_enable_prune(NeighborList& nl, cudaStream_t st);
+// Lists the groups that hold an atom whose type (caller frame) is negative, now
+// and at every build; null: no more (host sync; no work on the list queued).
+int nl_set_marks(NeighborList& nl, const int* type);
 // Entries of the batches that the last prune pass kept (host sync).
 int nl_kept_entries(NeighborList& nl, long long* kept, cudaStream_t st);
 // Update as NEIGHBOR_LIST::Update (neighbor_list.cpp:974-1025): forced, or
@@ -359,10 +366,16 @@ struct GroupArgs {
   // soft-core: state B table and parameters
   const float2* lj_b = nullptr;
   int n_types_b = 0;
+  const int* marked = nullptr;  // groups with a marked atom
+  const int* nmarked = nullptr;
   float lambda = 0.f, alp_A = 0.f, alp_B = 0.f, sigma6 = 0.f, sigma6_min = 0.f;
 };
+// (of a soft-core box, the rows of groups without a marked atom)
 int launch_pair_groups(GroupArgs a, Accumulators& acc, bool energy, bool virial,
                        cudaStream_t st);
+// The rows of groups with a marked atom (soft-core).
+int launch_marked_groups(GroupArgs a, Accumulators& acc, bool energy, bool virial,
+                         cudaStream_t st);
 
 // Rigid triangle: atoms A, B, C, canonical frame (A at (0, ra), B at (rc, rb),
 // C at (rd, re) about the centre of mass) and masses.

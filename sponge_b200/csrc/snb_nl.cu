@@ -521,6 +521,8 @@ struct GroupSearchArgs {
   int cap;
   unsigned* entry;
   int* flags;
+  const int* mark_type;       // caller frame, negative: marked; or null
+  const int* perm;
   BatchView bv;
 };
 
@@ -547,7 +549,10 @@ __device__ __forceinline__ float span_gap(int o, float lo, float hi) {
 // the cutoff of two i atoms: on liquid water at cutoff 10 A, skin 2 A, 80 of
 // the 116 (batch, atom) evaluations of a row remain, against 115 in the order
 // of the cells (the pair kernel: 161 us, against 167 us with 16 even bins and
-// 173 us with 10).
+// 173 us with 10).  Marked partners (soft-core) go to the first bin: sharing
+// batches, they leave a row near them few that need the soft-core terms (step
+// of 13,000 and 42,000 atoms with 30 and 52 marked sites 75 and 128 us, with
+// them anywhere in the row 95 and 137).
 //
 // What bounds it is the chain of one group: its loads, its batches one after
 // another and the sort.  Launches in us (under ncu, cold) on 648, 1,299,
@@ -831,8 +836,9 @@ __global__ void __launch_bounds__(32 * (W > kGroupSearchWarps ? W : kGroupSearch
         }
         if (hits != 0u) {
           const int slot = before + __popc(m & lt);
+          const bool marked = a.mark_type != nullptr && a.mark_type[a.perm[j]] < 0;
           se[slot] = ((unsigned)j << 8) | hits;
-          sb[slot] = (unsigned char)min(31, (int)(rmin * bin_scale));
+          sb[slot] = (unsigned char)(marked ? 0 : min(31, (int)(rmin * bin_scale)));
         }
         held = after;
         if (full != 0) {
@@ -875,9 +881,24 @@ __global__ void __launch_bounds__(32 * (W > kGroupSearchWarps ? W : kGroupSearch
   }
 }
 
+// The groups with a marked atom, in no particular order (flags null: whether or
+// not the list is being rebuilt).
+__global__ void k_list_marked(int ngroups, const int2* __restrict__ group,
+                              const int* __restrict__ perm, const int* __restrict__ type,
+                              int* __restrict__ list, int* count, const int* flags) {
+  if (flags && flags[kFlagNeed] == 0) return;
+  const int id = blockIdx.x * blockDim.x + threadIdx.x;
+  if (id >= ngroups) return;
+  const int2 g = group[id];
+  bool any = false;
+  for (int t = 0; t < g.y; ++t) any = any || type[perm[g.x + t]] < 0;
+  if (any) list[atomicAdd(count, 1)] = id;
+}
+
 // batch: a rebuild of only some systems keeps the total of the others
-__global__ void k_rebuild_begin(int* flags, bool batch) {
+__global__ void k_rebuild_begin(int* flags, bool batch, int* nmarked) {
   if (flags[kFlagNeed] == 0) return;
+  if (nmarked) *nmarked = 0;
   if (!batch || flags[kFlagFull] != 0) flags[kFlagTotal] = 0;
   flags[kFlagMaxRow] = 0;
 }
@@ -1245,6 +1266,8 @@ static void groups_free(NeighborList& nl) {
   cudaFree(nl.d_gpairs);
   cudaFree(nl.d_gentry);
   cudaFree(nl.d_gmask);
+  cudaFree(nl.d_marked);
+  nl.d_marked = nullptr;
   nl.d_atom_key = nl.d_grow_count = nl.d_gpairs = nullptr;
   nl.d_group = nullptr;
   nl.d_gentry = nullptr;
@@ -1271,6 +1294,10 @@ static int groups_alloc(NeighborList& nl, cudaStream_t st) {
   SNB_CUDA_TRY(cudaMalloc(&nl.d_gpairs, sizeof(int) * G));
   SNB_CUDA_TRY(cudaMemsetAsync(nl.d_gpairs, 0, sizeof(int) * G, st));
   SNB_CUDA_TRY(cudaMalloc(&nl.d_gentry, sizeof(unsigned) * G * nl.gcap));
+  if (nl.mark_type) {
+    SNB_CUDA_TRY(cudaMalloc(&nl.d_marked, sizeof(int) * G));
+    SNB_CUDA_TRY(cudaMemsetAsync(nl.d_nmarked, 0, sizeof(int), st));
+  }
   if (pruned) return nl_enable_prune(nl, st);
   return kOk;
 }
@@ -1363,8 +1390,22 @@ int nl_enable_prune(NeighborList& nl, cudaStream_t st) {
   return kOk;
 }
 
+int nl_set_marks(NeighborList& nl, const int* type) {
+  nl.mark_type = nullptr;
+  if (!type || !nl.groups) return kOk;
+  if (!nl.d_nmarked) SNB_CUDA_TRY(cudaMalloc(&nl.d_nmarked, sizeof(int)));
+  if (!nl.d_marked) SNB_CUDA_TRY(cudaMalloc(&nl.d_marked, sizeof(int) * nl.group_room));
+  SNB_CUDA_TRY(clear_now(nl.d_nmarked, sizeof(int)));
+  k_list_marked<<<ceil_div(nl.max_groups, 128), 128>>>(nl.max_groups, nl.d_group, nl.d_perm,
+                                                       type, nl.d_marked, nl.d_nmarked, nullptr);
+  SNB_CUDA_TRY(cudaStreamSynchronize(nullptr));
+  nl.mark_type = type;
+  return kOk;
+}
+
 void nl_free(NeighborList& nl) {
   groups_free(nl);
+  cudaFree(nl.d_nmarked);
   cudaFree(nl.d_prune_ref);
   cudaFree(nl.d_unsorted);
   cudaFree(nl.d_sorted_cell);
@@ -1548,7 +1589,8 @@ int nl_rebuild(NeighborList& nl, const float* crd_f, const int* atom_local,
                                                           nl.d_flags, need, cell_sys);
   else
     SNB_CUDA_TRY(cudaMemsetAsync(nl.d_cell_count, 0, sizeof(int) * nl.ncell, st));
-  k_rebuild_begin<<<1, 1, 0, st>>>(nl.d_flags, need != nullptr);
+  k_rebuild_begin<<<1, 1, 0, st>>>(nl.d_flags, need != nullptr,
+                                   nl.mark_type ? nl.d_nmarked : nullptr);
   int* key = nl.groups ? nl.d_atom_key : nullptr;
   if (nl.bv.nsys > 0)
     k_bin_count<true><<<ceil_div(n, 256), 256, 0, st>>>(
@@ -1611,6 +1653,8 @@ int nl_rebuild(NeighborList& nl, const float* crd_f, const int* atom_local,
     ga.cap = nl.gcap;
     ga.entry = nl.d_gentry;
     ga.flags = nl.d_flags;
+    ga.mark_type = nl.mark_type;
+    ga.perm = nl.d_perm;
     ga.bv = nl.bv;
     // (the warps per group: see k_group_search)
     const int per_sm = std::max(1, nl.search_blocks_per_sm);
@@ -1624,6 +1668,10 @@ int nl_rebuild(NeighborList& nl, const float* crd_f, const int* atom_local,
     const int gblocks = W == 1 ? std::min(ceil_div(nl.max_groups, kGroupSearchWarps), sms * per_sm)
                                : std::min(nl.max_groups, sms * 2 * per_sm);
     search<<<gblocks, 32 * std::max(W, kGroupSearchWarps), 0, st>>>(ga);
+    if (nl.mark_type)
+      k_list_marked<<<ceil_div(nl.max_groups, 128), 128, 0, st>>>(
+          nl.max_groups, nl.d_group, nl.d_perm, nl.mark_type, nl.d_marked, nl.d_nmarked,
+          nl.d_flags);
     k_finish_build<<<1, 1, 0, st>>>(nl.d_flags);
     if (need)  // the systems' flags for the next decision
       SNB_CUDA_TRY(cudaMemsetAsync(nl.bv.box_need, 0, nl.bv.nsys, st));
