@@ -151,6 +151,34 @@ __device__ __forceinline__ double warp_sum(double v) {
   return v;
 }
 
+constexpr float kTwoOverSqrtPi = 1.1283791670955126f;
+
+// LJ energy of a pair from r^-6 with the stored A' = 12 A, B' = 6 B.
+__device__ __forceinline__ float lj_energy(float A, float B, float ir6) {
+  return (0.083333333f * A * ir6 - 0.166666667f * B) * ir6;
+}
+// sigma^6 of the soft-core radius (LJ_soft_core.h:33-149).
+__device__ __forceinline__ float sc_sigma6(float A, float B, float s6, float s6min) {
+  return (A == 0.f || B == 0.f) ? s6 : fmaxf(0.5f * A / B, s6min);
+}
+
+// The polynomial of erfcx in t = 1 / (1 + x / 2), highest power first; mul_add
+// forms a t + b for the caller's type (one argument, or two at a time).
+template <typename T, typename MulAdd>
+__device__ __forceinline__ T erfcx_poly(T t, T first, MulAdd mul_add) {
+  T p = first;
+  p = mul_add(p, t, 0.33589873f);
+  p = mul_add(p, t, -0.88379663f);
+  p = mul_add(p, t, 1.0076897f);
+  p = mul_add(p, t, -0.39945206f);
+  p = mul_add(p, t, 0.47237507f);
+  p = mul_add(p, t, 0.22729602f);
+  p = mul_add(p, t, 0.2896666f);
+  p = mul_add(p, t, -0.00045567533f);
+  return p;
+}
+constexpr float kErfcxFirst = -0.049221702f;
+
 // erfc(x) and exp(-x^2) together for x >= 0.  erfcx(x) = erfc(x) e^{x^2} is
 // a degree-8 polynomial in t = 1/(1 + x/2) on [0, 4] (weighted least-squares
 // fit against double-precision erfcx; max relative error 3.3e-7 in float32), so
@@ -169,16 +197,7 @@ __device__ __forceinline__ float erfc_and_exp(float x, float* e_out) {
   const float e = __expf(-x * x);
   *e_out = e;
   const float t = __fdividef(1.0f, 1.0f + 0.5f * x);
-  float p = -0.049221702f;
-  p = fmaf(p, t, 0.33589873f);
-  p = fmaf(p, t, -0.88379663f);
-  p = fmaf(p, t, 1.0076897f);
-  p = fmaf(p, t, -0.39945206f);
-  p = fmaf(p, t, 0.47237507f);
-  p = fmaf(p, t, 0.22729602f);
-  p = fmaf(p, t, 0.2896666f);
-  p = fmaf(p, t, -0.00045567533f);
-  return p * e;
+  return erfcx_poly(t, kErfcxFirst, [](float a, float x, float b) { return fmaf(a, x, b); }) * e;
 }
 
 // atomicAdd(&counter[key], 1) with the lanes of a warp that share the same

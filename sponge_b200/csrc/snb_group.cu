@@ -31,7 +31,6 @@
 
 namespace snb {
 
-constexpr float kTwoOverSqrtPi = 1.1283791670955126f;
 constexpr int kGroupWarps = 4;
 constexpr float kFarAway = 1e15f;  // beyond every cutoff, its square finite
 
@@ -89,26 +88,13 @@ __device__ __forceinline__ float2 erfc_exp2(float2 r, float2 r2, const PairConst
   *ex = e;
   const float2 u = __ffma2_rn(r, both(c.half), both(1.0f));
   const float2 t = make_float2(rcp_fast(u.x), rcp_fast(u.y));
-  float2 p = both(-0.049221702f);
-  p = __ffma2_rn(p, t, both(0.33589873f));
-  p = __ffma2_rn(p, t, both(-0.88379663f));
-  p = __ffma2_rn(p, t, both(1.0076897f));
-  p = __ffma2_rn(p, t, both(-0.39945206f));
-  p = __ffma2_rn(p, t, both(0.47237507f));
-  p = __ffma2_rn(p, t, both(0.22729602f));
-  p = __ffma2_rn(p, t, both(0.2896666f));
-  p = __ffma2_rn(p, t, both(-0.00045567533f));
+  const float2 p = erfcx_poly(
+      t, both(kErfcxFirst), [](float2 a, float2 x, float b) { return __ffma2_rn(a, x, both(b)); });
   return __fmul2_rn(p, e);
 }
 
 // Soft-core pair forms (LJ_soft_core.h:33-149) of a pair whose end states
 // differ: force over r, LJ and Coulomb energies.
-__device__ __forceinline__ float sc_sigma6(float A, float B, float s6, float s6min) {
-  return (A == 0.f || B == 0.f) ? s6 : fmaxf(0.5f * A / B, s6min);
-}
-__device__ __forceinline__ float lj_energy(float A, float B, float ir6) {
-  return (0.083333333f * A * ir6 - 0.166666667f * B) * ir6;
-}
 __device__ __noinline__ void soft_terms(float lam, float alp_A, float alp_B, float s6,
                                         float s6min, float beta, float AA, float AB, float BA,
                                         float BB, float r2, float qq, float* fs, float* elj,

@@ -29,8 +29,6 @@
 
 namespace snb {
 
-constexpr float kTwoOverSqrtPi = 1.1283791670955126f;
-
 template <int ACCUM>
 __device__ __forceinline__ void add_force(Accumulators& acc, int s, float fx,
                                           float fy, float fz) {
@@ -113,7 +111,7 @@ __device__ __forceinline__ void lj_pair_ab(const Args& a, Accumulators& acc, flo
   if (ENERGY || VIRIAL) {
     const bool own_i = gi < a.global[j];
     if (ENERGY) {
-      const float elj = COUL_ONLY ? 0.f : (0.083333333f * A * ir6 - 0.166666667f * B) * ir6;
+      const float elj = COUL_ONLY ? 0.f : lj_energy(A, B, ir6);
       const float ec = qq * erfc_br * rinv;
       if (own_i) {
         e_lj += elj;
@@ -380,12 +378,6 @@ int launch_pair(const PairArgs& a, Accumulators& acc, int accum, bool energy,
 // pair uses the soft-core radius r_sc = (r^6 + alpha lambda^p sigma^6)^(1/6)
 // for state A and (r^6 + alpha (1-lambda)^p sigma^6)^(1/6) for state B, with
 // sigma^6 = max(A'/(2B'), sigma_min^6), or the input sigma^6 when A' or B' is 0.
-__device__ __forceinline__ float lj_e(float A, float B, float ir6) {
-  return (0.083333333f * A * ir6 - 0.166666667f * B) * ir6;
-}
-__device__ __forceinline__ float sc_sigma(float A, float B, float s6, float s6min) {
-  return (A == 0.f || B == 0.f) ? s6 : fmaxf(0.5f * A / B, s6min);
-}
 // dU/dlambda chain term (Get_Soft_Core_dU_dlambda, LJ_soft_core.h:142-149)
 __device__ __forceinline__ float sc_dudl(float F, float sigma, float rsc, float alpha,
                                          float p, float lambda) {
@@ -440,16 +432,16 @@ k_lj_soft(SoftArgs a, Accumulators acc, long long* dudl_total) {
       const float ir2 = 1.0f / r2, ir6 = ir2 * ir2 * ir2;
       fs = lam_ * (AB - AA * ir6) * ir6 * ir2 + lam * (BB - BA * ir6) * ir6 * ir2 -
            coul_f(qq, a.beta, r);
-      elj = lam_ * lj_e(AA, AB, ir6) + lam * lj_e(BA, BB, ir6);
+      elj = lam_ * lj_energy(AA, AB, ir6) + lam * lj_energy(BA, BB, ir6);
       ec = coul_e(qq, a.beta, r);
       if (DUDL) {
-        dl = lj_e(BA, BB, ir6) - lj_e(AA, AB, ir6);
+        dl = lj_energy(BA, BB, ir6) - lj_energy(AA, AB, ir6);
         const float dqj = a.dq ? a.dq[j] : 0.f;
         dc = erfcf(a.beta * r) * (dqj * pi.w + pj.w * dqi) / r;
       }
     } else {
-      const float sA = sc_sigma(AA, AB, a.sigma6, a.sigma6_min);
-      const float sB = sc_sigma(BA, BB, a.sigma6, a.sigma6_min);
+      const float sA = sc_sigma6(AA, AB, a.sigma6, a.sigma6_min);
+      const float sB = sc_sigma6(BA, BB, a.sigma6, a.sigma6_min);
       const float r6 = r2 * r2 * r2;
       const float rA = powf(r6 + alp_A * sA, 0.16666667f);
       const float rB = powf(r6 + alp_B * sB, 0.16666667f);
@@ -465,9 +457,9 @@ k_lj_soft(SoftArgs a, Accumulators acc, long long* dudl_total) {
                         (expf(-bB * bB) * kTwoOverSqrtPi * a.beta + erfcf(bB) / rB) * iB6;
       fs = lam_ * flA + lam * flB - (lam_ * fcA + lam * fcB);
       ec = lam_ * coul_e(qq, a.beta, rA) + lam * coul_e(qq, a.beta, rB);
-      elj = lam_ * lj_e(AA, AB, iA6) + lam * lj_e(BA, BB, iB6);
+      elj = lam_ * lj_energy(AA, AB, iA6) + lam * lj_energy(BA, BB, iB6);
       if (DUDL) {
-        dl = lj_e(BA, BB, iB6) - lj_e(AA, AB, iA6);
+        dl = lj_energy(BA, BB, iB6) - lj_energy(AA, AB, iA6);
         dl += sc_dudl((AB - AA * iA6) * iA6 * iA2, sA, rA, a.alpha, a.p, lam) -
               sc_dudl((BB - BA * iB6) * iB6 * iB2, sB, rB, a.alpha, a.p, lam_);
         const float dqj = a.dq ? a.dq[j] : 0.f;
