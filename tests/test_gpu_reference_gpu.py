@@ -4,6 +4,7 @@ fixed-point engine on the same 9,000-atom box: both against the FP64 oracle,
 and a short NVE run of each from the same start."""
 
 import copy
+import os
 
 import numpy as np
 import pytest
@@ -21,7 +22,9 @@ def g():
 
 @pytest.fixture(scope="module")
 def refgpu(g, box_9k):
-    from oracle.oracle import ReferenceGPU
+    from oracle.oracle import REF_GPU_SO, ReferenceGPU
+    if not os.path.exists(REF_GPU_SO):
+        pytest.skip("reference GPU build not present")
     r = ReferenceGPU()
     r.init(box_9k, 8.0, 2.0)
     return r
