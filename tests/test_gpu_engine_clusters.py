@@ -1,17 +1,17 @@
-"""The engine's cluster form of the neighbor list.
+"""The engine's list at sizes the other files leave out, and the calls kept for
+the two forms it had earlier.
 
-On request a single rectangular box with at least five cells per axis runs
-on clusters (up to four atoms of a cell, each neighbour cluster stored once
-per cluster with its 4x4 pair mask) instead of the default rows.  Held
-here:
+snb_engine_set_list_form chose between a row per atom and clusters of four;
+both values now give the grouped rows, and the value is stored and given back.
+Held here, with the value 1 set:
   * the pair set is the oracle's FP32 pair set bit for bit (the reference's
     criterion, exclusions, each pair once), at two cutoffs, with atoms
     far outside the box (unwrapped images) and with random positions;
-  * forces, energies and virials of both list forms are within 1e-5 / 1e-6
-    of FP64, and within 1e-6 of each other;
+  * forces, energies and virials are within 1e-5 / 1e-6 of FP64, equal for
+    both values, and within 1e-6 of the modules' row kernel;
   * graph-replayed MD steps equal stream-launched ones bit for bit, and a
     list that outgrows its rows is regrown and the steps repeated;
-  * boxes below five cells per axis keep the rows.
+  * the value 1 is refused where clusters were (below five cells per axis).
 """
 
 import ctypes
@@ -30,7 +30,7 @@ def g():
     return gpu_helpers
 
 
-def _clusters(g, e):
+def _set_form(g, e):
     g.capi.check(g.capi.load().snb_engine_set_list_form(e, 1), "set_list_form")
     return _form(g, e)
 
@@ -74,7 +74,7 @@ def test_cluster_pair_set_bit_exact(g, oracle, box_9k, cutoff):
     s = box_9k
     e = g.engine_create(s, cutoff)
     try:
-        assert _clusters(g, e) == 1
+        assert _set_form(g, e) == 1
         _force(g, e, s)
         got = _pairs(g, e)
     finally:
@@ -94,7 +94,7 @@ def test_cluster_pair_set_unwrapped_and_random(g, oracle):
     s.crd[100:400] = (rng.random((300, 3)) * s.box).astype(np.float32)  # overlaps
     e = g.engine_create(s, 7.0, skin=1.5)
     try:
-        assert _clusters(g, e) == 1
+        assert _set_form(g, e) == 1
         _force(g, e, s)
         got = _pairs(g, e)
     finally:
@@ -123,7 +123,20 @@ def test_forms_agree_with_fp64_and_each_other(g, oracle, box_9k):
             assert abs(t[idx] - en[k]) <= 2e-6 * abs(en[k]), (form, k)
         scale = np.abs(vir).max()
         assert np.abs(t[8:14] - vir).max() <= 2e-6 * scale, form
-    assert g.rel_rms(out[1][0], out[0][0]) <= 1e-6
+    assert np.array_equal(out[1][0], out[0][0]) and np.array_equal(out[1][1], out[0][1])
+    # the modules: a row per atom, the same FP32 pair terms in another order
+    box = g.Box(s)
+    nl, lj = g.make_nl(box, 8.0, 2.0), g.lj_create(box, 8.0)
+    pme, beta, _ = g.pme_create(box, 8.0)
+    try:
+        g.nl_update(nl, box)
+        rows = (g.lj_force(lj, nl, box, beta)["frc"] + g.pme_excluded(pme, box)["frc"] +
+                g.pme_reciprocal(pme, box)["frc"])
+    finally:
+        lib.snb_nl_destroy(nl)
+        lib.snb_lj_destroy(lj)
+        lib.snb_pme_destroy(pme)
+    assert g.rel_rms(out[0][0], rows) <= 1e-6
 
 
 def _md(g, e, s, steps, graph, first=0):
@@ -150,7 +163,7 @@ def test_graph_equals_stream_on_clusters(g, box_9k):
         e = g.engine_create(s, 8.0)
         g.engine_set_water_bonded(e, s)
         try:
-            assert _clusters(g, e) == 1
+            assert _set_form(g, e) == 1
             res.append(_md(g, e, s, 120, graph))
         finally:
             g.capi.load().snb_engine_destroy(e)
@@ -169,7 +182,7 @@ def test_dense_region_regrows_cluster_rows(g, oracle):
     s.crd[:, 0] = np.where(x < L / 2, x * np.float32(0.5), x)  # left half squeezed
     e = g.engine_create(s, 8.0)
     try:
-        assert _clusters(g, e) == 1
+        assert _set_form(g, e) == 1
         _force(g, e, s)
         got = _pairs(g, e)
     finally:
@@ -179,6 +192,7 @@ def test_dense_region_regrows_cluster_rows(g, oracle):
 
 
 def test_small_box_uses_rows(g, small_box):
+    """(The value 1 is refused there, as clusters were.)"""
     lib = g.capi.load()
     e = g.engine_create(small_box, 8.0)
     try:
