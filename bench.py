@@ -1117,9 +1117,13 @@ def run_ours(args):
         if "ns_per_day" in plain:
             plain["speedup_vs_plain"] = plain["this_engine_ns_per_day"] / plain["ns_per_day"]
 
-    # roofline of the dominant kernel (the pair kernel), HBM view.  Per
-    # launch: the grouped rows' entries that the last prune pass kept (4 bytes
-    # each; a pass takes about a quarter more), the positions, types and forces
+    # the dominant kernel (the pair kernel).  What bounds it is instruction issue
+    # and its latencies (66 % issue active, no pipe above 40 %: the committed
+    # counters); the fraction given is of the measured HBM peak, which it is far
+    # below.  Bytes per launch: the grouped rows' entries that the last prune
+    # pass kept (4 bytes each; a pass takes about a quarter more; without prune
+    # passes all entries, one for about 5 listed pairs), the positions, types
+    # and forces
     pair_ms = float(phases[2])
     listed = int(pairs.value)
     prof_prunes = int(pq1.value - pq0.value)
@@ -1128,12 +1132,15 @@ def run_ours(args):
     peak, peak_kind = measured_peaks()
     achieved = alg_bytes / (pair_ms * 1e-3) / 1e9
     traffic = committed_traffic()
-    roofline = {"bound": "hbm", "kernel": "k_lj_groups", "achieved": achieved,
+    roofline = {"bound": "issue", "kernel": "k_lj_groups", "achieved": achieved,
                 "peak": peak, "peak_kind": peak_kind, "unit": "GB/s",
                 "frac": achieved / peak,
                 "traffic": (traffic["dram_bytes_per_launch"] if traffic else None),
                 "algorithmic_bytes": alg_bytes, "kernel_ms": pair_ms,
-                "entries_scanned_per_launch": scanned, "prune_passes_profiled": prof_prunes,
+                "entries_scanned_per_launch": scanned,
+                "entries_scanned_kind": ("kept by the last prune pass" if kept.value > 0 else
+                                         "estimated: listed pairs / 5"),
+                "prune_passes_profiled": prof_prunes,
                 "profiled_steps": args.profile_steps}
     # FP32-pipe view: 47 flops per in-cutoff pair (force only) + 10 per other
     # pair of an entry and the about seven atoms of its group; in-cutoff count

@@ -17,6 +17,13 @@
 // (cutoff 10 A, skin 2 A) the launch takes 150 us, where the row kernel with
 // pruned rows took 187 us; on the 1M-atom soft-core box 1.28-1.34 ms against
 // 1.95-2.03 ms; on 64 boxes of 200-2,000 waters 208 us against 280 us.
+//
+// A partner's force is summed over the group's atoms in 32 bits (two chains of
+// four) and added once in 64, an i atom's along the lanes' shares of its row;
+// energies and virials go to 64 bits after at most eight pairs.  The error of
+// the forces against 64 bits over 30 boxes of 600 to 39,000 atoms is 0.99 of
+// the row kernel's (geometric mean; median 1.01, 0.5 to 1.4).
+//
 // Five blocks of four warps per SM (96 registers): four blocks 158 us, six
 // (spilling) 158 us.  Four i atoms at a time 158-164 us; the polynomial on
 // unpaired FMAs 153 us; rows handed out by an atomic counter 170-180 us (the

@@ -9,14 +9,18 @@
 // dropped when gj is in the exclusion list of gi (:744-803).
 //
 // The layout is different.  Atoms are counting-sorted into cells of side
-// L/floor(L/((cutoff+skin)/2)) with a stable order inside each cell (caller
-// index), so the sorted order and the list are deterministic.  One warp scans,
-// for one sorted atom i, the atoms after i in its own cell and the neighbor
-// cells its cell owns (+-2 cells), walked as runs of consecutive cells along
-// z: each run is one contiguous slice of the sorted coordinate array, read
-// with coalesced 16-byte loads, and is trimmed to the cells whose box comes
-// within rl of atom i.  Hits go in one pass into rows of fixed capacity;
-// a row that would overflow raises a flag and the host regrows the rows.
+// L/floor(L/((cutoff+skin)/2)) with a fixed order inside each cell, so the
+// sorted order and the list are deterministic.  A cell owns half of its
+// neighbor cells (+-2 cells), walked as runs of consecutive cells along z:
+// each run is one contiguous slice of the sorted coordinate array, read with
+// coalesced 16-byte loads, and is trimmed to the cells whose box comes within
+// rl.  The list has two forms.  The modules keep a row per atom
+// (k_pair_search: one warp scans, for one sorted atom i, the atoms after i in
+// its own cell and the runs; order inside a cell by caller index).  The engine
+// keeps a row per group of up to eight atoms of a cell (k_group_search; order
+// inside a cell along a path up and down its quarter columns).  Either is
+// written in one pass into rows of fixed capacity; a row that would overflow
+// raises a flag and the host regrows the rows.
 #include <algorithm>
 #include <cfloat>
 #include <cmath>
