@@ -101,6 +101,7 @@ def _check(g, oracle, s, cutoff, tol=1e-5):
 @pytest.mark.parametrize("waters,cutoff,tol", [
     (200, 8.0, 1e-5),    # half the box 9.07 A: every pair imaged, 3 cells per axis
     (231, 9.0, 1e-5),    # the cutoff just below half the box
+    (200, 10.0, 1e-5),   # the cutoff beyond half the box: nearest images only
     (700, 7.3, 1e-5),    # 5 cells per axis: trimmed runs, some groups imaged
     (1500, 9.0, 1e-9),   # beta * cutoff = 4.3: beyond the polynomial
     (2600, 6.1, 1e-5),   # narrow cells: groups of a few atoms
@@ -111,6 +112,32 @@ def test_groups_match_fp64(g, oracle, waters, cutoff, tol):
     from sponge_b200 import systems
     s = systems.water_box(waters, seed=waters, ion_pairs=None)
     _check(g, oracle, s, cutoff, tol)
+
+
+@pytest.mark.parametrize("waters", [1, 2, 5])
+def test_smallest_boxes(g, oracle, waters):
+    """One group or a few, in a box of empty cells.  A water's excluded and
+    reciprocal forces on itself nearly cancel (each about 4 kcal/mol/A, their
+    sum 0.03), so the error is held to the terms' sizes: 1e-5 of them, the
+    reciprocal part going through a float FFT and a grid in steps of 2^-22
+    (up to 6e-6 of its size against FP64 on a full box)."""
+    from sponge_b200 import systems
+    s = dataclasses.replace(systems.water_box(waters, seed=2), box=26.0)
+    lib = g.capi.load()
+    e = g.engine_create(s, 8.0)
+    try:
+        got = _force_of(g, e, g.dev(s.crd.reshape(-1), np.float32), s.n, 0)
+        pairs = _pairs(g, e)
+    finally:
+        lib.snb_engine_destroy(e)
+    rs, cols = oracle.nl_pairs_system(s, 8.0, 2.0)
+    assert np.array_equal(pairs, g.csr_to_pairs(rs, cols))
+    beta = oracle.get_beta(8.0)
+    terms = [oracle.direct_f64(s, 8.0, beta, rs, cols)["frc"],
+             oracle.excluded_f64(s, beta)["frc"],
+             oracle.pme_f64(s, (systems.fft_size(s.box),) * 3, beta)["frc"]]
+    size = sum(np.linalg.norm(t) for t in terms)
+    assert np.linalg.norm(got - sum(terms)) <= 1e-5 * size
 
 
 def test_long_rows_of_a_large_box(g, oracle):
