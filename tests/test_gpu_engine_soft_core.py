@@ -75,6 +75,44 @@ def test_engine_soft_core_matches_fp64(g, oracle, soft_box, lam):
     assert t[1] == pytest.approx(f / V, rel=1e-6)
 
 
+@pytest.mark.parametrize("marked", ["every water", "no atom"])
+def test_engine_soft_core_marks(g, oracle, soft_box, marked):
+    """The rows of groups with an atom whose end states differ run by
+    themselves: all rows (state B has another LJ for the water oxygens too), or
+    none (state B is state A)."""
+    import torch
+    from sponge_b200 import systems
+    s, sc = soft_box
+    if marked == "every water":
+        sc = dataclasses.replace(sc, BA=sc.BA * np.float32(1.1), BB=sc.BB * np.float32(1.05))
+    else:
+        sc = dataclasses.replace(sc, type_B=sc.type_A, n_types_B=sc.n_types_A, BA=sc.AA, BB=sc.AB)
+    lib = g.capi.load()
+    box = g.Box(s)
+    e = g.engine_create(s, CUTOFF)
+    h = g.soft_create(box, sc, CUTOFF, _params(0.5))
+    crd = g.dev(s.crd.reshape(-1), np.float32)
+    frc = torch.zeros(3 * s.n, dtype=torch.float32, device="cuda")
+    tot = torch.zeros(16, dtype=torch.float64, device="cuda")
+    try:
+        g.capi.check(lib.snb_engine_set_soft_core(e, h), "set_soft_core")
+        g.capi.check(lib.snb_engine_force(e, g.ptr(crd), g.ptr(frc), 0, 1, 1, g.ptr(tot),
+                                          g.stream()), "engine_force")
+        torch.cuda.synchronize()
+    finally:
+        lib.snb_engine_destroy(e)
+        lib.snb_lj_soft_destroy(h)
+    beta = oracle.get_beta(CUTOFF)
+    rs, cols = oracle.nl_pairs_system(s, CUTOFF, 2.0)
+    d = oracle.soft_f64(s, sc, CUTOFF, beta, 0.5, 0.5, 1.0, 3.0, 0.0, rs, cols)
+    want = (d["frc"] + oracle.excluded_f64(s, beta)["frc"] +
+            oracle.pme_f64(s, (systems.fft_size(s.box),) * 3, beta)["frc"])
+    assert g.rel_rms(frc.cpu().numpy().reshape(-1, 3), want) <= 1e-5
+    t = tot.cpu().numpy()
+    for idx, key in ((0, "lj_energy"), (2, "coulomb_energy")):
+        assert abs(t[idx] - d[key].sum()) <= 2e-6 * np.abs(d[key]).sum(), key
+
+
 def test_engine_soft_core_md_runs(g, soft_box):
     """20 graph-replayed NVE steps with soft-core pair terms at lambda 0.5 stay
     finite and match the same steps launched on the stream bit for bit."""
