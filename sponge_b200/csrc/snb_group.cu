@@ -526,10 +526,14 @@ static int multiprocessors() {
 int launch_marked_groups(GroupArgs a, Accumulators& acc, bool energy, bool virial,
                          cudaStream_t st) {
   if (a.n <= 0) return kOk;
-  const int blocks = std::min(ceil_div((long long)a.ngroups << 4, kGroupWarps),
-                              multiprocessors());
   GroupKern kern = group_kernel(a, kMarkedRows, energy, virial);
   leave_shared_memory(kern);
+  // all resident blocks: the marked groups may be all of them (every water's LJ
+  // changed, 28,000 waters: step 251 us, with one block per SM 613)
+  int per_sm = 1;
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32 * kGroupWarps, 0);
+  const int blocks = std::min(ceil_div((long long)a.ngroups << 4, kGroupWarps),
+                              multiprocessors() * std::max(per_sm, 1));
   kern<<<blocks, 32 * kGroupWarps, 0, st>>>(a, acc);
   SNB_CUDA_TRY(cudaGetLastError());
   return kOk;
