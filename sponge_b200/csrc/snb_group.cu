@@ -178,10 +178,9 @@ __device__ __forceinline__ float2 image2(float2 d, float L, float rL) {
 // atom, or those with one.  Nearly all pairs of a marked row take the soft-core
 // terms, so one such row by one warp outlasts the rest of the launch on boxes
 // of less than 50,000 atoms: the marked rows have a launch of their own beside
-// the others, in parts of about a batch (step of 7,500, 19,200, 38,000 and
-// 300,000 atoms with 35 to 64 marked sites: 56, 100, 114 and 594 us, in one
-// launch with whole rows 78, 112, 137 and 599; marked rows in parts at the
-// start of one launch, with more registers spilled: -, 98, 116 and 620).
+// the others, in parts of about a batch (step of 19,200, 42,000 and 300,000
+// atoms with 35 to 64 marked sites: 89, 116 and 565 us, in one launch with whole
+// rows 112, 159 and 599).
 enum { kNoSoft, kPlainRows, kMarkedRows };
 
 template <bool ENERGY, bool VIRIAL, bool BATCH, int SOFT, bool FAR>
